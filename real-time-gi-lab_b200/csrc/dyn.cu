@@ -113,7 +113,10 @@ __global__ void __launch_bounds__(256) k_dyn_alloc(DynDev d, VoxDev v) {
   uint32_t tot;
   uint32_t ex = block_scan_256(c, &tot);
   __shared__ uint32_t s_pre;
-  if (threadIdx.x == 0) s_pre = chain_prefix(d.look, blk, tot, d.hdr + 6);   // a give-up sets header word 12
+  if (threadIdx.x < 32u) {
+    const uint32_t pre = chain_prefix(d.look, blk, tot, d.hdr + 6);   // a give-up sets header word 12
+    if (threadIdx.x == 0) s_pre = pre;
+  }
   __syncthreads();
   const uint32_t excl = s_pre + ex;
   if (w >= nw) return;

@@ -63,28 +63,40 @@ __device__ __forceinline__ uint32_t chain_ticket(unsigned long long *look) {
   return t;
 }
 
-// One thread per block: publishes part k's sum, looks back for its exclusive prefix, publishes the inclusive prefix.
+// One whole warp per block: publishes part k's sum, looks back for its exclusive prefix, publishes the inclusive prefix.
+// The lanes read 32 predecessors at a time, lane l the part l + 1 before the last one not yet counted, so a look-back over
+// n parts costs n / 32 round trips to L2 (one thread walking them one by one made a 5120-part scan 98 us).
 // hold = k + 1 makes part k publish nothing (a test of the bounded wait: the parts after it give up), else 0.
 __device__ __forceinline__ uint32_t chain_prefix(unsigned long long *look, uint32_t k, uint32_t sum, uint32_t *hdr,
                                                  uint32_t hold = 0u) {
+  const uint32_t lane = threadIdx.x & 31u;
   if (hold != 0u && hold == k + 1u) return 0u;
   unsigned long long *st = look + 1;
-  if (k == 0u) { st_release_u64(st, (2ull << 32) | sum); return 0u; }
-  st_release_u64(st + k, (1ull << 32) | sum);
-  uint32_t excl = 0, j = k - 1u, spins = 0;
-  for (;;) {
-    unsigned long long x = ld_acquire_u64(st + j);
-    uint32_t f = (uint32_t)(x >> 32);
-    if (f == 0u) {
-      if (++spins > LOOK_SPIN) { atomicExch(&hdr[6], 1u); break; }
+  if (k == 0u) {
+    if (lane == 0u) st_release_u64(st, (2ull << 32) | sum);
+    return 0u;
+  }
+  if (lane == 0u) st_release_u64(st + k, (1ull << 32) | sum);
+  uint32_t excl = 0, spins = 0;
+  for (int j = (int)k - 1;;) {
+    const int q = j - (int)lane;
+    const unsigned long long x = q >= 0 ? ld_acquire_u64(st + q) : 2ull << 32;   // before part 0: an empty prefix
+    const uint32_t f = (uint32_t)(x >> 32);
+    const uint32_t ready = __ballot_sync(0xffffffffu, f != 0u), full = __ballot_sync(0xffffffffu, f == 2u);
+    const uint32_t need = full ? full ^ (full - 1u) : 0xffffffffu;   // the lanes up to the nearest inclusive prefix
+    if ((ready & need) != need) {
+      if (++spins > LOOK_SPIN) {
+        if (lane == 0u) atomicExch(&hdr[6], 1u);
+        break;
+      }
       __nanosleep(32);
       continue;
     }
-    excl += (uint32_t)x;
-    if (f == 2u || j == 0u) break;
-    j--;
+    excl += __reduce_add_sync(0xffffffffu, (need >> lane) & 1u ? (uint32_t)x : 0u);
+    if (full) break;
+    j -= 32;
   }
-  st_release_u64(st + k, (2ull << 32) | (excl + sum));
+  if (lane == 0u) st_release_u64(st + k, (2ull << 32) | (excl + sum));
   return excl;
 }
 

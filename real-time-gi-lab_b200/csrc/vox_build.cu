@@ -190,9 +190,9 @@ __device__ __forceinline__ void mark_one(const VoxDev &v, const Tri &T, uint32_t
 }
 
 // clear (voxel.ts:338-344)
-__global__ void k_clear(VoxDev v) {
+__global__ void k_clear(VoxDev v, uint32_t parts) {
   grid_dep_wait();
-  uint32_t n = v.levels * v.G * v.G * v.G, nl = v.scan_cap + 1u;
+  uint32_t n = v.levels * v.G * v.G * v.G, nl = parts + 1u;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n || i < GI_HDR || i < nl; i += gridDim.x * blockDim.x) {
     if (i < GI_HDR) v.hdr[i] = 0u;
     if (i < 4u) v.work[i] = 0u;
@@ -266,49 +266,93 @@ __global__ void __launch_bounds__(256, 4) k_mark_bricks_big(VoxDev v, SceneDev s
 
 // ---- ordered allocation of the marked bricks (countMarks / scanMarks / allocBricks, voxel.ts:411-470) ---------------
 // Order space o in [0, levels * G^3): level levels-1 first, pointer index within a level.
-// The ordered brick allocation takes 256 * k pointer entries per block, k per thread: k = 1 unless the block sums
-// would not fit the scan buffer (alloc_per_thread)
-
 __device__ __forceinline__ uint32_t order_to_ptr(uint32_t o, uint32_t per, uint32_t NL) {
   return (NL - 1u - o / per) * per + o % per;
 }
 
 // allocBricks (voxel.ts:411-470: countMarks, scanMarks, allocBricks) in the fixed order, one pass: each block takes
-// 256 * kpt consecutive entries of the order space, kpt per thread.
-__global__ void __launch_bounds__(256) k_alloc_bricks(VoxDev v, uint32_t kpt, uint32_t nblocks) {
+// 256 E consecutive entries of the order space, each warp 32 E of them as rows of 32 W, a lane W = min(E, 4) at a time (128-bit
+// loads for W = 4 where the pointers are aligned; a level holds a multiple of 64 entries, so a lane's four never straddle two
+// levels).  The rows' counts (at most 128 each) are scanned over the warp packed in one word's bytes.  The per-level counts go
+// through shared memory: one atomic per block and level.  Bound by latency: the launch, the look-back's round trips and, with
+// few blocks, each thread's own entries; E balances the last two (gi_launch_vox_build).  A 5 x 512^3 clipmap (1.3 M pointers)
+// takes 11.4 us where 256 pointers a block and a one-thread look-back took 98 us, a 4 x 128^3 one (16,384) 5.6 against 10.8.
+template <uint32_t E>
+__global__ void __launch_bounds__(256) k_alloc_bricks(VoxDev v, uint32_t nblocks) {
   grid_dep_wait();
-  uint32_t per = v.G * v.G * v.G, NL = v.levels, n = NL * per, G = v.G;
-  uint32_t blk = chain_ticket(v.look);
-  uint32_t o0 = blk * 256u * kpt;
-  uint32_t flags = 0, c = 0;
-  for (uint32_t k = 0; k < kpt; k++) {
-    uint32_t o = o0 + threadIdx.x * kpt + k;
-    bool m = o < n && v.ptr[order_to_ptr(o, per, NL)] == GI_MARK;
-    flags |= (m ? 1u : 0u) << k;
-    c += m ? 1u : 0u;
+  constexpr uint32_t W = E < 4u ? E : 4u, ROWS = E / W;
+  __shared__ uint32_t s_warp[8], s_pre, s_level[8], s_drop;
+  const uint32_t per = v.G * v.G * v.G, NL = v.levels, n = NL * per, G = v.G;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  if (threadIdx.x < 8u) s_level[threadIdx.x] = 0u;
+  if (threadIdx.x == 8u) s_drop = 0u;
+  const uint32_t blk = chain_ticket(v.look);
+  const uint32_t o0 = blk * 256u * E + wid * 32u * E + lane * W;
+  const bool wide = (reinterpret_cast<size_t>(v.ptr) & 15u) == 0u;
+  uint32_t flags = 0, cnt = 0;   // W bits and one byte per row
+#pragma unroll
+  for (uint32_t k = 0; k < ROWS; k++) {
+    const uint32_t o = o0 + k * 32u * W;
+    if (o >= n) continue;
+    const uint32_t *p = v.ptr + order_to_ptr(o, per, NL);
+    uint32_t f;
+    if (W == 1u) {
+      f = p[0] == GI_MARK ? 1u : 0u;
+    } else {
+      uint4 q;
+      if (wide) q = *reinterpret_cast<const uint4 *>(p);
+      else q = make_uint4(p[0], p[1], p[2], p[3]);
+      f = (q.x == GI_MARK ? 1u : 0u) | (q.y == GI_MARK ? 2u : 0u) | (q.z == GI_MARK ? 4u : 0u) | (q.w == GI_MARK ? 8u : 0u);
+    }
+    flags |= f << (W * k);
+    cnt |= (uint32_t)__popc(f) << (8u * k);
   }
-  uint32_t tot;
-  uint32_t ex = block_scan_256(c, &tot);
-  __shared__ uint32_t s_pre;
-  if (threadIdx.x == 0) {
-    uint32_t pre = chain_prefix(v.look, blk, tot, v.hdr, v.scan_hold);
-    s_pre = pre;
-    if (blk == nblocks - 1u) { v.hdr[0] = pre + tot; v.hdr[5] = pre + tot; }
+  uint32_t inc = cnt;   // inclusive over the lanes
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= (uint32_t)d) inc += y;
+  }
+  const uint32_t rows = __shfl_sync(0xffffffffu, inc, 31), ex = inc - cnt;
+  if (lane == 0u) s_warp[wid] = (rows & 255u) + ((rows >> 8) & 255u) + ((rows >> 16) & 255u) + (rows >> 24);
+  __syncthreads();
+  if (wid == 0u) {
+    const uint32_t tot = __reduce_add_sync(0xffffffffu, lane < 8u ? s_warp[lane] : 0u);
+    const uint32_t pre = chain_prefix(v.look, blk, tot, v.hdr, v.scan_hold);
+    if (lane == 0u) {
+      s_pre = pre;
+      if (blk == nblocks - 1u) { v.hdr[0] = pre + tot; v.hdr[5] = pre + tot; }
+    }
   }
   __syncthreads();
-  ex += s_pre;
-  for (uint32_t k = 0; k < kpt; k++) {
-    if (!((flags >> k) & 1u)) continue;
-    uint32_t o = o0 + threadIdx.x * kpt + k;
-    uint32_t i = order_to_ptr(o, per, NL);
-    uint32_t idx = ex++;
-    if (idx >= v.max_bricks) { v.ptr[i] = GI_DROP; atomicAdd(&v.hdr[2], 1u); continue; }
-    uint32_t L = i / per, r = i % per;
-    atomicAdd(&v.hdr[8 + L], 1u);
-    v.ptr[i] = idx;
-    v.base[idx] = 0u;
-    v.code[idx] = (L << 27) | ((r % G) << 18) | (((r / G) % G) << 9) | (r / (G * G));
+  if (flags != 0u) {
+    uint32_t first = s_pre;
+    for (uint32_t w = 0; w < wid; w++) first += s_warp[w];
+#pragma unroll
+    for (uint32_t k = 0; k < ROWS; k++) {
+      const uint32_t f = (flags >> (W * k)) & ((1u << W) - 1u);
+      if (f != 0u) {
+        uint32_t idx = first + ((ex >> (8u * k)) & 255u), kept = 0u, dropped = 0u;
+        const uint32_t i0 = order_to_ptr(o0 + k * 32u * W, per, NL), L = i0 / per;
+#pragma unroll
+        for (uint32_t j = 0; j < W; j++) {
+          if (!((f >> j) & 1u)) continue;
+          const uint32_t i = i0 + j, r = i - L * per, at = idx++;
+          if (at >= v.max_bricks) { v.ptr[i] = GI_DROP; dropped++; continue; }
+          v.ptr[i] = at;
+          v.base[at] = 0u;
+          v.code[at] = (L << 27) | ((r % G) << 18) | (((r / G) % G) << 9) | (r / (G * G));
+          kept++;
+        }
+        if (kept) atomicAdd(&s_level[L], kept);
+        if (dropped) atomicAdd(&s_drop, dropped);
+      }
+      first += (rows >> (8u * k)) & 255u;
+    }
   }
+  __syncthreads();
+  if (threadIdx.x < 8u && s_level[threadIdx.x]) atomicAdd(&v.hdr[8 + threadIdx.x], s_level[threadIdx.x]);
+  if (threadIdx.x == 8u && s_drop) atomicAdd(&v.hdr[2], s_drop);
 }
 
 // The rest of the brick init and clearKeys (voxel.ts:467, :471-474): zero the occupancy (64 B) and representatives
@@ -485,14 +529,14 @@ __device__ __forceinline__ bool voxel_takes(const VoxDev &v, const SceneDev &s, 
 // voxBitsBig (voxel.ts:515-534), balanced: one warp per chunk of a big item, taken from a queue (big_chunks cut the
 // items); then one warp per item listed with chunks past the table, from its first untabulated chunk to its end.  The
 // lanes' occupancy bits are ORed per word inside the warp (neighbouring cells share a word), one atomic per word.
-__global__ void __launch_bounds__(256, 4) k_vox_bits_big(VoxDev v, SceneDev s) {
+__global__ void __launch_bounds__(256, 4) k_vox_bits_big(VoxDev v, SceneDev s, uint32_t parts) {
   grid_dep_wait();
   uint32_t lane = threadIdx.x & 31u;
   uint32_t bo = v.hdr[2];
   const uint32_t tab = min(v.work[2], v.citem_cap);   // chunks found through the table
   const uint32_t work = tab + v.work[3];               // + the listed items
   // the attribute allocation's chained scan (the brick allocation's is done)
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= v.scan_cap; q += gridDim.x * blockDim.x) v.look[q] = 0ull;
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= parts; q += gridDim.x * blockDim.x) v.look[q] = 0ull;
   for (;;) {
     uint32_t ch = 0;
     if (lane == 0) ch = atomicAdd(&v.work[1], 1u);
@@ -631,7 +675,10 @@ __global__ void __launch_bounds__(256) k_alloc_voxels(VoxDev v, uint32_t nblocks
   uint32_t tot;
   uint32_t ex = block_scan_256(c, &tot);
   __shared__ uint32_t s_pre;
-  if (threadIdx.x == 0) s_pre = chain_prefix(v.look, blk, tot, v.hdr);
+  if (threadIdx.x < 32u) {
+    const uint32_t pre = chain_prefix(v.look, blk, tot, v.hdr);
+    if (threadIdx.x == 0) s_pre = pre;
+  }
   __syncthreads();
   uint32_t first = ex + s_pre;
   if (b < nb) {
@@ -739,19 +786,22 @@ using namespace gi;
 cudaError_t gi_launch_vox_build(const VoxDev &v, const SceneDev &s, uint32_t sm_count, cudaStream_t st) {
   uint32_t per = v.G * v.G * v.G, nptr = v.levels * per;
   uint32_t persist = sm_count * v.blocks;   // blocks of 256 threads per SM for the grid-stride passes (default 8)
-  GI_TRY(gi_launch(k_clear, min((nptr + 255u) / 256u + 1u, persist), 256, st, v));
+  // Pointers per thread of the brick allocation: 1 while the parts are at most one look-back step (32 parts), 4 to some 500
+  // parts, 16 above (measured: 512 pointers 4.2 us with 1, 8.5 with 16; 16,384: 6.0 with 1, 5.6 with 4, 9.2 with 16; 163,840:
+  // 10.6 with 1, 8.0 with 4; 1.3 M: 11.4 with 16).  The parts of both chained scans fit the scan words, allotted for 256 a part.
+  const uint32_t E = nptr <= 8192u ? 1u : (nptr <= 524288u ? 4u : 16u);
+  const uint32_t ab = (nptr + 256u * E - 1u) / (256u * E), vb = (v.max_bricks + VOX_CHUNK - 1u) / VOX_CHUNK;
+  GI_TRY(gi_launch(k_clear, min((nptr + 255u) / 256u + 1u, persist), 256, st, v, ab));
   uint32_t tb = (s.threads + 255u) / 256u;   // threads of the triangle passes (the work items' triangles)
   if (tb) GI_TRY(gi_launch(k_mark_bricks, tb, 256, st, v, s));
   GI_TRY(gi_launch(k_mark_bricks_big, persist, 256, st, v, s));
-  uint32_t kpt = 1;
-  while ((nptr + 256u * kpt - 1u) / (256u * kpt) > v.scan_cap && kpt < 32u) kpt *= 2u;
-  uint32_t ab = (nptr + 256u * kpt - 1u) / (256u * kpt);
-  GI_TRY(gi_launch(k_alloc_bricks, ab, 256, st, v, kpt, ab));
+  if (E == 1u) GI_TRY(gi_launch(k_alloc_bricks<1u>, ab, 256, st, v, ab));
+  else if (E == 4u) GI_TRY(gi_launch(k_alloc_bricks<4u>, ab, 256, st, v, ab));
+  else GI_TRY(gi_launch(k_alloc_bricks<16u>, ab, 256, st, v, ab));
   GI_TRY(gi_launch(k_init_bricks, persist, 256, st, v));
   if (tb) GI_TRY(gi_launch(k_vox_bits, tb, 256, st, v, s));
-  GI_TRY(gi_launch(k_vox_bits_big, persist, 256, st, v, s));
+  GI_TRY(gi_launch(k_vox_bits_big, persist, 256, st, v, s, vb));
   if (v.levels > 1) GI_TRY(gi_launch(k_reduce, persist, 256, st, v));
-  uint32_t vb = (v.max_bricks + VOX_CHUNK - 1u) / VOX_CHUNK;
   GI_TRY(gi_launch(k_alloc_voxels, vb, 256, st, v, vb));
   GI_TRY(gi_launch(k_resolve_attr, persist, 256, st, v, s));
   return cudaGetLastError();

@@ -299,9 +299,9 @@ __device__ __forceinline__ void w_compact(const RcDev &r, const VoxDev &v, const
   uint32_t tot;
   const uint32_t ex = block_scan_256(mine, &tot);
   __shared__ uint32_t s_pre, s_over;
-  if (threadIdx.x == 0) {
-    s_pre = chain_prefix(look, blk, tot, w.state + 1);   // a give-up sets state[7]
-    s_over = 0u;
+  if (threadIdx.x < 32u) {
+    const uint32_t pre = chain_prefix(look, blk, tot, w.state + 1);   // a give-up sets state[7]
+    if (threadIdx.x == 0) { s_pre = pre; s_over = 0u; }
   }
   __syncthreads();
   const uint32_t first = s_pre + ex;
