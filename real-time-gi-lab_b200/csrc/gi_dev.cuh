@@ -119,6 +119,24 @@ __device__ __forceinline__ float gi_exp(float x) {
   return p * __int_as_float((int)(k + 127.0f) << 23);
 }
 
+// x / b per component for a divisor shared by many quotients, r = RN(1 / b): the same bits as dividing.  The product x r is
+// corrected twice by its remainder with fused multiply-adds; after the first correction the quotient is within one ulp, and
+// the second then rounds correctly (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990: the remainder is exact and r correctly rounded).  That needs the remainders clear of
+// the subnormals: b in [2^-40, 2^40] (the caller's), every component +0 or in [2^-80, 2^60]; others are divided.
+__device__ __forceinline__ float div_step(float x, float b, float r) {
+  const float q0 = x * r;
+  const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, x), r, q0);
+  return __fmaf_rn(__fmaf_rn(-q1, b, x), r, q1);
+}
+__device__ __forceinline__ f3 div_shared(f3 x, float b, float r) {
+  const uint32_t ux = __float_as_uint(x.x), uy = __float_as_uint(x.y), uz = __float_as_uint(x.z);
+  // +0 wraps to the largest; a sign bit makes the largest too large
+  if (min(min(ux - 1u, uy - 1u), uz - 1u) >= 0x17800000u - 1u && max(max(ux, uy), uz) <= 0x5d800000u)
+    return mk(div_step(x.x, b, r), div_step(x.y, b, r), div_step(x.z, b, r));
+  return x / b;
+}
+
 // ---- WGSL packing builtins (public WGSL spec formulas) -------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack4x8unorm(float a, float b, float c, float d) {
   float v[4] = {a, b, c, d};

@@ -646,50 +646,78 @@ __device__ __forceinline__ void sh_basis(f3 n, float y[9]) {
 }
 
 // projectSH (rc.ts:752-774) of cascade-0 probe pi, fused into its merge: the probe's 16 directions (res 4) are held by
-// its four quad threads, four consecutive lanes, 4 merged radiances each (as stored).  Every lane of the group collects
-// the 16 with shuffles and sums the 27 coefficients over the directions in order 0..15, with fused multiply-adds; lane
-// i of the group stores the probe's coefficient groups 2i and 2i+1.
+// its four quad threads, four consecutive lanes, 4 merged radiances each (as stored).  Lane i of the group takes the 16
+// radiances of colour channel i (the fourth lane repeats the third's) and sums that channel's 9 coefficients over the
+// directions in order 0..15, with fused multiply-adds; then lane i collects and stores coefficient groups 2i and 2i+1.
+// All lanes of the warp call it; `on`: the group has a probe.
 template <int A>
-__device__ __forceinline__ void project_sh_quads(const RcDev &r, uint32_t pi, const f3 mr[4]) {
-  const uint32_t lane = threadIdx.x & 31u, gbase = lane & ~3u;
-  const unsigned gmask = 0xFu << gbase;
+__device__ __forceinline__ void project_sh_quads(const RcDev &r, uint32_t pi, bool on, const f3 mr[4]) {
+  const uint32_t lane = threadIdx.x & 31u, gbase = lane & ~3u, ch = lane & 3u;
   const float *F = r.frame;
-  f3 cf[9];
+  float cf[9];
 #pragma unroll
-  for (int k = 0; k < 9; k++) cf[k] = mk(0.0f, 0.0f, 0.0f);
+  for (int k = 0; k < 9; k++) cf[k] = 0.0f;
 #pragma unroll
   for (uint32_t d = 0; d < 16u; d++) {
     const uint32_t u = d & 3u, vr = d >> 2, j = (vr & 1u) * 2u + (u & 1u);
     const int src = (int)(gbase + (vr >> 1) * 2u + (u >> 1));
-    f3 rd = mk(__shfl_sync(gmask, mr[j].x, src), __shfl_sync(gmask, mr[j].y, src), __shfl_sync(gmask, mr[j].z, src));
-    f3 rr = rd * F[F_OMEGA + d];
-    float4 dv = r.dirs[r.c[0].dir_off + d];   // dirOf(d, 4), tabulated
+    const float x = __shfl_sync(0xffffffffu, mr[j].x, src), y1 = __shfl_sync(0xffffffffu, mr[j].y, src),
+                z = __shfl_sync(0xffffffffu, mr[j].z, src);
+    const float rr = (ch == 0u ? x : (ch == 1u ? y1 : z)) * F[F_OMEGA + d];
+    const float4 dv = r.dirs[r.c[0].dir_off + d];   // dirOf(d, 4), tabulated (tabulating the basis too was no faster)
     float y[9];
     sh_basis(mk(dv.x, dv.y, dv.z), y);
 #pragma unroll
-    for (int k = 0; k < 9; k++) cf[k] = fma3(rr, y[k], cf[k]);
+    for (int k = 0; k < 9; k++) cf[k] = __fmaf_rn(rr, y[k], cf[k]);
   }
-  float vals[32];
-#pragma unroll
-  for (int k = 0; k < 32; k++) vals[k] = 0.0f;
   const float a0 = GI_PI, a1 = 2.0f * GI_PI / 3.0f, a2 = GI_PI / 4.0f;
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    float a = k == 0 ? a0 : (k < 4 ? a1 : a2);
-    vals[k * 3 + 0] = cf[k].x * a; vals[k * 3 + 1] = cf[k].y * a; vals[k * 3 + 2] = cf[k].z * a;
-  }
+  for (int k = 0; k < 9; k++) cf[k] = cf[k] * (k == 0 ? a0 : (k < 4 ? a1 : a2));
+  float vals[32];
+#pragma unroll
+  for (int q = 0; q < 32; q++) vals[q] = q < 27 ? __shfl_sync(0xffffffffu, cf[q / 3], (int)gbase + q % 3) : 0.0f;
   typedef typename Atlas<A>::T T;
 #pragma unroll
   for (uint32_t q = 0; q < 8u; q++) {
-    if ((q >> 1) != (lane & 3u)) continue;
+    if (!on || (q >> 1) != ch) continue;
     float4 val = make_float4(vals[4 * q], vals[4 * q + 1], vals[4 * q + 2], vals[4 * q + 3]);
     if (r.f32_out) reinterpret_cast<float4 *>(r.sh)[(size_t)pi * 8u + q] = val;
     else Atlas<A>::store(reinterpret_cast<T *>(r.sh), (size_t)pi * 8u + q, val);
   }
 }
 
-// mergeScreen (rc.ts:710-743) for cascade c, in place, one 2x2 quad of directions (four rays) per thread.  The four
-// upper probes and their weights depend only on the probe, so a thread computes them once for its four rays.
+// The upper cascade's weighted mean for the quad's four rays (those whose interval is not opaque): src the texels of upper
+// probe 0 at the quad's first direction, 2^log2 texels a probe, res a row.  ws the sum of the valid probes' weights, rws its
+// reciprocal; 0 without a valid probe.
+template <int A>
+__device__ __forceinline__ void merge_up(const typename Atlas<A>::T *__restrict__ src, uint32_t log2, uint32_t res, const float4 vv[4],
+                                         const float w[4], const uint32_t qi[4], float ws, float rws, f3 up[4]) {
+#pragma unroll
+  for (uint32_t j = 0; j < 4; j++) {
+    if (!(vv[j].w > 0.0f)) continue;
+    float4 p[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+      p[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (qi[k] != GI_EMPTY) p[k] = Atlas<A>::load(src, ((size_t)qi[k] << log2) + (j >> 1) * res + (j & 1u));
+    }
+    f3 acc = mk(0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if (qi[k] != GI_EMPTY) acc = fma3(mk(p[k].x, p[k].y, p[k].z), w[k], acc);
+    up[j] = mk(0.0f, 0.0f, 0.0f);
+    // the weights are at least 1e-8 and at most 1.0002 each
+    if (ws >= 1e-9f && ws <= 8.0f) up[j] = div_shared(acc, ws, rws);
+    else if (ws > 0.0f) up[j] = acc / ws;
+  }
+}
+
+// mergeScreen (rc.ts:710-743) for cascade c, in place, one 2x2 quad of directions (four rays) per thread; whole warps call
+// it.  The four upper probes and their weights depend only on the probe: of a warp's quads (8 probes' in cascade 0, 2 in
+// cascade 1, one above) lane 4 p + k weighs upper probe k of the warp's probe p, and the quads take them by shuffles.  The
+// branch on the upper resolution stands outside the rays, and the four means divide by one sum (div_shared: an IEEE division
+// is some 25 instructions, and there were twelve).  Bound by latency (37 % issue-active in a wave that does not fill the chip):
+// 1290 -> 700 warp instructions per 32 quads, the colonnade's five merges 59 -> 41 us, a 641 x 361 view's 45 -> 24.
 // upperAvg (rc.ts:681-686) of the upper cascade comes from up_avg, the quad averages the upper cascade's merge wrote
 // from its stored (rounded) texels: the same four values summed in the same order, so the same bits.  When this
 // cascade's resolution is twice the lower one's, the thread writes its own quad's average for the merge below.
@@ -699,80 +727,78 @@ __device__ __forceinline__ void merge_quad(const RcDev &r, uint32_t c, uint32_t 
   typedef typename Atlas<A>::T T;
   T *rad = reinterpret_cast<T *>(r.rad);
   const CascDev &L = r.c[c];
-  uint32_t hr = L.res >> 1, hq_log2 = L.dirs_log2 - 2u;   // quads per row, log2 quads per probe
-  if (t >= (L.np << hq_log2)) return;
-  uint32_t pi = t >> hq_log2, qd = t & ((1u << hq_log2) - 1u);
-  uint32_t u0 = (qd % hr) * 2u, v0 = (qd / hr) * 2u;
+  const uint32_t hq = L.dirs_log2 - 2u, hr_log2 = L.dirs_log2 / 2u - 1u;   // log2 quads per probe, per row
+  const uint32_t n = L.np << hq, lane = threadIdx.x & 31u, t0 = t - lane;
+  if (t0 >= n) return;   // the whole warp
+  const bool on = t < n;
+  const uint32_t pi = (on ? t : n - 1u) >> hq, qd = t & ((1u << hq) - 1u);
+  const uint32_t u0 = (qd & ((1u << hr_log2) - 1u)) * 2u, v0 = (qd >> hr_log2) * 2u;
   const float *F = r.frame;
   const bool has_up = c + 1u < r.cascades;
-  bool pr_ok = false;
-  float w[4];
-  uint32_t qi[4];
-  bool qok[4];
-  if (has_up) {
-    ProbeDev pr = r.probes[L.probe_off + pi];
-    pr_ok = pr.pos.w > 0.0f;
-    if (pr_ok) {
-      const CascDev &U = r.c[c + 1u];
-      float cx = ((float)(pi % L.tiles_x) + 0.5f) * (float)L.tile_size;
-      float cy = ((float)(pi / L.tiles_x) + 0.5f) * (float)L.tile_size;
-      float ux = div_tile(cx, U) - 0.5f, uy = div_tile(cy, U) - 0.5f;
-      int bx = __float2int_rd(ux), by = __float2int_rd(uy);
-      float fx = ux - (float)bx, fy = uy - (float)by;
+  const size_t idx0 = (size_t)L.rad_off + ((size_t)pi << L.dirs_log2) + v0 * L.res + u0;
+  float4 vv[4];
 #pragma unroll
-      for (uint32_t k = 0; k < 4; k++) {
-        int ox = (int)(k & 1u), oy = (int)(k >> 1);
-        int qx = iclamp(bx + ox, 0, (int)U.tiles_x - 1), qy = iclamp(by + oy, 0, (int)U.tiles_y - 1);
-        qi[k] = (uint32_t)qy * U.tiles_x + (uint32_t)qx;
-        ProbeDev qp = r.probes[U.probe_off + qi[k]];
-        qok[k] = qp.pos.w > 0.0f;
-        float fwx = ox == 1 ? fx : 1.0f - fx, fwy = oy == 1 ? fy : 1.0f - fy;
-        float rel = fabsf(qp.nrm.w - pr.nrm.w) / pr.nrm.w;
-        w[k] = (fwx * fwy + 1e-4f) * (gi_exp(-20.0f * rel) + 1e-4f);
+  for (uint32_t j = 0; j < 4; j++)   // (0,0) (1,0) (0,1) (1,1): upperAvg's a, b, c, d order
+    vv[j] = Atlas<A>::load(rad, idx0 + (j >> 1) * L.res + (j & 1u));
+  float w[4], ws = 0.0f;
+  uint32_t qi[4];   // the upper probes; GI_EMPTY: not valid
+  if (has_up) {
+    const CascDev &U = r.c[c + 1u];
+    const uint32_t sh = min(hq, 5u), mine = (t0 >> hq) + (lane >> 2);
+    float wk = 0.0f;
+    uint32_t qk = GI_EMPTY;
+    if ((lane >> 2) < (32u >> sh) && mine < L.np) {
+      const ProbeDev &pr = r.probes[L.probe_off + mine];
+      if (pr.pos.w > 0.0f) {
+        const float z = pr.nrm.w;
+        const uint32_t py = mine / L.tiles_x, px = mine - py * L.tiles_x;
+        const float cx = ((float)px + 0.5f) * (float)L.tile_size, cy = ((float)py + 0.5f) * (float)L.tile_size;
+        const float ux = div_tile(cx, U) - 0.5f, uy = div_tile(cy, U) - 0.5f;
+        const int bx = __float2int_rd(ux), by = __float2int_rd(uy);
+        const float fx = ux - (float)bx, fy = uy - (float)by;
+        const int ox = (int)(lane & 1u), oy = (int)((lane >> 1) & 1u);
+        const int qx = iclamp(bx + ox, 0, (int)U.tiles_x - 1), qy = iclamp(by + oy, 0, (int)U.tiles_y - 1);
+        const uint32_t q = (uint32_t)qy * U.tiles_x + (uint32_t)qx;
+        const ProbeDev &qp = r.probes[U.probe_off + q];
+        if (qp.pos.w > 0.0f) {
+          qk = q;
+          const float fwx = ox == 1 ? fx : 1.0f - fx, fwy = oy == 1 ? fy : 1.0f - fy;
+          const float rel = fabsf(qp.nrm.w - z) / z;
+          wk = (fwx * fwy + 1e-4f) * (gi_exp(-20.0f * rel) + 1e-4f);
+        }
       }
     }
+    const uint32_t src = (lane >> sh) << 2;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+      w[k] = __shfl_sync(0xffffffffu, wk, (int)(src + k));
+      qi[k] = __shfl_sync(0xffffffffu, qk, (int)(src + k));
+      if (qi[k] != GI_EMPTY) ws += w[k];
+    }
+  }
+  f3 up[4];
+#pragma unroll
+  for (uint32_t j = 0; j < 4; j++) up[j] = mk(F[F_SKY], F[F_SKY + 1], F[F_SKY + 2]);
+  if (has_up) {
+    const CascDev &U = r.c[c + 1u];
+    const float rws = 1.0f / ws;
+    if (U.res == L.res) merge_up<A>(rad + U.rad_off + (v0 * U.res + u0), U.dirs_log2, U.res, vv, w, qi, ws, rws, up);
+    else merge_up<GI_ATLAS_F32>(up_avg + (v0 * L.res + u0), L.dirs_log2, L.res, vv, w, qi, ws, rws, up);
   }
   f3 qsum = mk(0.0f, 0.0f, 0.0f);
   f3 mr[4];   // the four merged radiances as stored (rounded to the atlas)
 #pragma unroll
-  for (uint32_t j = 0; j < 4; j++) {   // (0,0) (1,0) (0,1) (1,1): upperAvg's a, b, c, d order
-    uint32_t u = u0 + (j & 1u), v = v0 + (j >> 1);
-    size_t idx = (size_t)L.rad_off + ((size_t)pi << L.dirs_log2) + v * L.res + u;
-    float4 vv = Atlas<A>::load(rad, idx);
-    f3 up = mk(F[F_SKY], F[F_SKY + 1], F[F_SKY + 2]);
-    if (has_up && vv.w > 0.0f) {
-      up = mk(0.0f, 0.0f, 0.0f);
-      if (pr_ok) {
-        const CascDev &U = r.c[c + 1u];
-        f3 acc = mk(0.0f, 0.0f, 0.0f);
-        float ws = 0.0f;
-#pragma unroll
-        for (uint32_t k = 0; k < 4; k++) {
-          if (!qok[k]) continue;
-          f3 ua;
-          if (U.res == L.res) {
-            float4 p = Atlas<A>::load(rad, (size_t)U.rad_off + ((size_t)qi[k] << U.dirs_log2) + v * U.res + u);
-            ua = mk(p.x, p.y, p.z);
-          } else {
-            float4 p = up_avg[((size_t)qi[k] << L.dirs_log2) + v * L.res + u];
-            ua = mk(p.x, p.y, p.z);
-          }
-          acc = fma3(ua, w[k], acc);
-          ws += w[k];
-        }
-        if (ws > 0.0f) up = acc / ws;
-      }
-    }
-    f3 m = fma3(up, vv.w, mk(vv.x, vv.y, vv.z));
-    Atlas<A>::store(rad, idx, make_float4(m.x, m.y, m.z, 1.0f));
+  for (uint32_t j = 0; j < 4; j++) {
+    const f3 m = fma3(up[j], vv[j].w, mk(vv[j].x, vv[j].y, vv[j].z));
+    if (on) Atlas<A>::store(rad, idx0 + (j >> 1) * L.res + (j & 1u), make_float4(m.x, m.y, m.z, 1.0f));
     mr[j] = mk(Atlas<A>::round(m.x), Atlas<A>::round(m.y), Atlas<A>::round(m.z));
     if (my_avg) qsum = qsum + mr[j];
   }
-  if (my_avg) {
-    f3 a = qsum * 0.25f;
-    my_avg[((size_t)pi << hq_log2) + (v0 >> 1) * hr + (u0 >> 1)] = make_float4(a.x, a.y, a.z, 0.0f);
+  if (my_avg && on) {
+    const f3 a = qsum * 0.25f;
+    my_avg[((size_t)pi << hq) + qd] = make_float4(a.x, a.y, a.z, 0.0f);
   }
-  if (c == 0u) project_sh_quads<A>(r, pi, mr);
+  if (c == 0u) project_sh_quads<A>(r, pi, on, mr);
 }
 
 template <int A>
