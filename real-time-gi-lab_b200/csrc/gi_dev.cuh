@@ -298,12 +298,14 @@ struct VoxDev {
   uint32_t *base;      // max_bricks first attribute
   uint32_t *code;      // max_bricks level << 27 | bx << 18 | by << 9 | bz
   uint32_t *rep;       // max_bricks * 512 representative triangle + 1 (build temporary)
-  uint32_t *big;       // 16 * big_cap big-triangle lists (build temporary)
+  uint32_t *big;       // 16 * big_cap big-triangle lists (build temporary; the last 8 hold the mark lists, then the medium items
+                       // from the front and the items listed whole from the back)
   uint4 *attr;         // max_voxels: albedo, normal, emissive rg, emissive b (one 16-byte load per hit)
   float *plane;        // max_voxels
   float *sunvis;       // max_voxels
   uint32_t *vpre;      // build temporary: max_bricks + 1 exclusive prefix of the bricks' voxel counts
-  uint32_t *work;      // build temporary: 4 words, the big-triangle queues, the chunk total, the items listed whole
+  uint32_t *work;      // build temporary: 4 words: markBricksBig's queue, then the medium items; voxBitsBig's queue; the chunk
+                       // total; the items listed whole
   uint32_t *cpre;      // build temporary: 8 * big_cap, per voxBits big-list slot its item's first chunk
   uint32_t *citem;     // build temporary (optional): the big-list slot of each chunk, citem_cap entries
   unsigned long long *look;   // build temporary: scan_cap + 1 words, the chained scans' ticket and block states

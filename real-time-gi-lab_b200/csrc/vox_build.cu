@@ -7,8 +7,8 @@
 //    can produce; they make the whole state deterministic, so the GPU state equals the oracle's word for word.
 //  * the representative-table clear (clearKeys) zeroes every allocated brick in one full-grid pass;
 //  * indirect dispatches (writeArgs) become grid-stride loops that read the device-side counts;
-//  * the big-triangle passes run one warp per (triangle, level) (markBricksBig) or per chunk of one (voxBitsBig), taken
-//    from a queue, instead of one 64-wide workgroup; resolveAttr runs one thread per voxel;
+//  * the big-triangle passes run one warp per (triangle, level) (markBricksBig), per chunk of one or per group of the smaller
+//    ones (voxBitsBig), taken from a queue, instead of one 64-wide workgroup; resolveAttr runs one thread per voxel;
 //  * markParents is folded into markBrick: the thread that marks a brick marks its ancestors;
 //  * list appends are warp-aggregated atomics.
 #include <cuda_runtime.h>
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(256) k_init_bricks(VoxDev v) {
   uint32_t nb = min(v.hdr[0], v.max_bricks);
   uint4 z = make_uint4(0u, 0u, 0u, 0u);
   uint4 *occ = reinterpret_cast<uint4 *>(v.occ), *rep = reinterpret_cast<uint4 *>(v.rep);
-  if (blockIdx.x == 0 && threadIdx.x == 0) v.work[1] = 0u;   // the voxBitsBig item counter
+  if (blockIdx.x == 0 && threadIdx.x == 0) { v.work[0] = 0u; v.work[1] = 0u; }   // the medium items, the voxBitsBig queue
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nb * 132u; q += gridDim.x * blockDim.x) {
     if (q < nb * 4u) occ[q] = z;
     else rep[q - nb * 4u] = z;
@@ -431,7 +431,11 @@ __device__ __forceinline__ void voxelize_one(const VoxDev &v, const SceneDev &s,
   atomicMax(&v.rep[ri], t + 1u);
 }
 
-// The big items' work for k_vox_bits_big: every big (triangle, level) of voxBits is cut into chunks of
+// Big items of at most this many cells go to k_vox_bits_big in groups (vox_medium), larger ones in chunks
+// (a cylinder facet of 44 cells, the colonnade's usual one, does better as a chunk of its own: 29 us against 37 with 64 here)
+constexpr uint32_t VOX_MEDIUM = 32, MEDIUM_GROUP = 8;
+
+// The large items' work for k_vox_bits_big: every (triangle, level) of voxBits with more cells is cut into chunks of
 // 2^chunk_log2 cells (a wall triangle clipped to a window covers ~10^4 cells; one warp per triangle left one warp working
 // long after the rest).  The warp reserves its items' chunks with one atomic, item after item; the item's first chunk
 // goes to cpre[slot] and, below citem_cap, the slot of every chunk to citem (written by the whole warp).  An item with
@@ -454,7 +458,7 @@ __device__ __forceinline__ void big_chunks(const VoxDev &v, uint32_t slot, uint3
   const uint32_t first = base + incl - nch;
   if (nch != 0u) {
     v.cpre[slot] = first;
-    if (first + nch > v.citem_cap) v.big[8u * v.big_cap + atomicAdd(&v.work[3], 1u)] = slot;
+    if (first + nch > v.citem_cap) v.big[16u * v.big_cap - 1u - atomicAdd(&v.work[3], 1u)] = slot;   // from the end down
   }
   for (uint32_t m = __ballot_sync(0xffffffffu, nch != 0u); m != 0u; m &= m - 1u) {
     const int src = __ffs(m) - 1;
@@ -489,15 +493,19 @@ __global__ void __launch_bounds__(256, 4) k_vox_bits(VoxDev v, SceneDev s) {
     }
     uint32_t k = warp_append(&v.hdr[16 + L], big);
     uint32_t slot = 0, nch = 0;
+    bool medium = false;
     if (big) {
       if (k < v.big_cap) {
         slot = L * v.big_cap + k;
         v.big[slot] = t;
-        nch = ((uint32_t)n + (1u << v.chunk_log2) - 1u) >> v.chunk_log2;
+        medium = (uint32_t)n <= VOX_MEDIUM;
+        if (!medium) nch = ((uint32_t)n + (1u << v.chunk_log2) - 1u) >> v.chunk_log2;
       } else {
         atomicAdd(&v.hdr[3], 1u);
       }
     }
+    const uint32_t km = warp_append(&v.work[0], medium);
+    if (medium) v.big[8u * v.big_cap + km] = slot;   // the mark lists' segments are free by now
     big_chunks(v, slot, nch);
     SmallItem it;
     it.T = T; it.t = t; it.r = r; it.n = n;
@@ -526,15 +534,88 @@ __device__ __forceinline__ bool voxel_takes(const VoxDev &v, const SceneDev &s, 
   return true;
 }
 
+// A group of medium items (9 .. VOX_MEDIUM cells) by one warp: lane i < MEDIUM_GROUP loads item i of the group, its triangle and
+// range, into shared memory; the group's cells are then dealt out 32 at a time over the warp, the owner of a cell found by its
+// prefix.  One warp per item spent its time on the item (five dependent loads, a range and the queue for one row of cells,
+// half empty); here up to eight items share them.  Bound by the box tests' issue and latency (66 % issue-active): voxBitsBig of
+// 200k triangles 88 -> 61 us, of the bounce scene's 120k 81 -> 63, of the colonnade 43 -> 29.  A warp takes about 1 us per row,
+// so groups of 8 for every scene made small ones wait on one warp (a room's 13 us became 38): the group grows with the items.
+struct MediumItem { float4 ab, bc, c_; int4 lo; int4 n; };   // a b c and the key; lo and L; nx, ny, 1 / nx, 1 / ny
+__device__ __forceinline__ void vox_medium(const VoxDev &v, const SceneDev &s, uint32_t g0, uint32_t items, uint32_t bo,
+                                           MediumItem *__restrict__ it) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t cells = 0;
+  if (lane < items) {
+    const uint32_t slot = v.big[8u * v.big_cap + g0 + lane], L = slot / v.big_cap, t = v.big[slot];
+    const Tri T = load_tri(s, t);
+    const Range r = vox_range(v, T, L, false);
+    cells = (uint32_t)(r.n.x * r.n.y * r.n.z);
+    it[lane].ab = make_float4(T.a.x, T.a.y, T.a.z, T.b.x);
+    it[lane].bc = make_float4(T.b.y, T.b.z, T.c.x, T.c.y);
+    it[lane].c_ = make_float4(T.c.z, __uint_as_float(t), __uint_as_float(T.idx.w), 0.0f);
+    it[lane].lo = make_int4(r.lo.x, r.lo.y, r.lo.z, (int)L);
+    it[lane].n = make_int4(r.n.x, r.n.y, __float_as_int(1.0f / (float)r.n.x), __float_as_int(1.0f / (float)r.n.y));
+  }
+  uint32_t incl = cells;
+#pragma unroll
+  for (uint32_t d = 1; d < MEDIUM_GROUP; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d && lane < MEDIUM_GROUP) incl += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, MEDIUM_GROUP - 1u);
+  __syncwarp();
+  for (uint32_t base = 0; base < total; base += 32u) {
+    const uint32_t g = base + lane;
+    uint32_t o = 0;
+#pragma unroll
+    for (uint32_t bit = MEDIUM_GROUP / 2u; bit >= 1u; bit >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, (int)(o + bit - 1u)) <= g) o += bit;
+    const uint32_t start = __shfl_sync(0xffffffffu, incl - cells, (int)o);
+    uint32_t wi = 0xffffffffu, msk = 0u, ri = 0u, key = 0u;
+    bool ok = false;
+    if (g < total) {
+      const float4 ab = it[o].ab, bc = it[o].bc, cc = it[o].c_;
+      const int4 lo = it[o].lo, n = it[o].n;
+      Tri T;
+      T.a = mk(ab.x, ab.y, ab.z); T.b = mk(ab.w, bc.x, bc.y); T.c = mk(bc.z, bc.w, cc.x);
+      key = __float_as_uint(cc.y);
+      T.idx = make_uint4(0u, 0u, 0u, __float_as_uint(cc.z));
+      // q / nx and (q / nx) / ny for q < VOX_MEDIUM: (q + 1/2) / n is at least 1 / (2 n) from an integer, far more than the
+      // product's rounding
+      const uint32_t q = g - start;
+      const int qy = (int)(((float)q + 0.5f) * __int_as_float(n.z)), z = (int)(((float)qy + 0.5f) * __int_as_float(n.w));
+      if (s.masked) {   // the alpha test samples the texture: it needs the vertices' indices
+        const uint4 idx = load_tri(s, key).idx;
+        T.idx = idx;
+      }
+      ok = voxel_takes(v, s, T, (uint32_t)lo.w, mki(lo.x + (int)q - qy * n.x, lo.y + qy - z * n.y, lo.z + z), bo, wi, msk, ri);
+    }
+    if (__ballot_sync(0xffffffffu, ok) == 0u) continue;
+    const uint32_t grp = __match_any_sync(0xffffffffu, ok ? wi : 0xffffffffu);
+    const uint32_t m = __reduce_or_sync(grp, msk);
+    if (ok) {
+      if ((uint32_t)(__ffs(grp) - 1) == lane) atomicOr(&v.occ[wi], m);
+      atomicMax(&v.rep[ri], key + 1u);
+    }
+  }
+  __syncwarp();   // the next group's items overwrite these
+}
+
 // voxBitsBig (voxel.ts:515-534), balanced: one warp per chunk of a big item, taken from a queue (big_chunks cut the
 // items); then one warp per item listed with chunks past the table, from its first untabulated chunk to its end.  The
 // lanes' occupancy bits are ORed per word inside the warp (neighbouring cells share a word), one atomic per word.
 __global__ void __launch_bounds__(256, 4) k_vox_bits_big(VoxDev v, SceneDev s, uint32_t parts) {
   grid_dep_wait();
+  __shared__ MediumItem s_item[8][MEDIUM_GROUP];
   uint32_t lane = threadIdx.x & 31u;
   uint32_t bo = v.hdr[2];
+  constexpr uint32_t MEDIUM_PER_WARP = 2u;   // the grid holds about twice the resident warps
   const uint32_t tab = min(v.work[2], v.citem_cap);   // chunks found through the table
-  const uint32_t work = tab + v.work[3];               // + the listed items
+  const uint32_t walked = tab + v.work[3];             // + the listed items
+  // medium items per group: 1 while that leaves warps without work, up to MEDIUM_GROUP where there are several per warp
+  const uint32_t med = v.work[0], spare = med * MEDIUM_PER_WARP / (gridDim.x * (blockDim.x >> 5));
+  const uint32_t group = spare >= 8u ? 8u : (spare >= 4u ? 4u : (spare >= 2u ? 2u : 1u));
+  const uint32_t work = walked + (med + group - 1u) / group;
   // the attribute allocation's chained scan (the brick allocation's is done)
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= parts; q += gridDim.x * blockDim.x) v.look[q] = 0ull;
   for (;;) {
@@ -542,8 +623,12 @@ __global__ void __launch_bounds__(256, 4) k_vox_bits_big(VoxDev v, SceneDev s, u
     if (lane == 0) ch = atomicAdd(&v.work[1], 1u);
     ch = __shfl_sync(0xffffffffu, ch, 0);
     if (ch >= work) break;
+    if (ch >= walked) {
+      vox_medium(v, s, (ch - walked) * group, min(group, med - (ch - walked) * group), bo, s_item[threadIdx.x >> 5]);
+      continue;
+    }
     const bool whole = ch >= tab;
-    const uint32_t slot = whole ? v.big[8u * v.big_cap + (ch - tab)] : v.citem[ch];
+    const uint32_t slot = whole ? v.big[16u * v.big_cap - 1u - (ch - tab)] : v.citem[ch];
     const uint32_t first = v.cpre[slot];
     const uint32_t part = whole ? max(first, v.citem_cap) - first : ch - first;
     const uint32_t L = slot / v.big_cap, t = v.big[slot];
