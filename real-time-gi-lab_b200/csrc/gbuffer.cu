@@ -10,9 +10,9 @@
 //
 // Binned in 16 x 16 pixel tiles: k_rs_setup gives every triangle its screen box, tile range and a depth bound,
 // k_rs_bin lists each triangle in the tiles its box touches (count, scan, fill), and one block per tile keeps its
-// 256 pixels' keys in registers while it walks the tile's list front to back by depth bound, in sorted chunks of 256.
-// A triangle whose bound is below the depth every pixel of the tile already holds cannot win anywhere in the tile
-// and ends the chunk; below one pixel's depth it is skipped for that pixel.  Skipped pairs are exactly pairs whose
+// 256 pixels' keys while it goes through the tile's list in chunks of 256, a chunk's large triangles front to back by
+// depth bound, then its small ones pixel by pixel.  A triangle whose bound is below the depth every pixel of the tile
+// already holds cannot win anywhere in the tile; below one pixel's depth it is skipped for that pixel.  Skipped pairs are exactly pairs whose
 // key would lose, so the result equals testing every (pixel, triangle whose box holds it) pair.  Triangles beyond the
 // list capacity go to an overflow list that every tile walks, so the result never depends on the capacity.
 #include <cuda_runtime.h>
@@ -177,12 +177,34 @@ __global__ void __launch_bounds__(256) k_rs_scan(uint32_t nblk, RasterDev rd) {
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_rs_bin(uint32_t ntris, uint32_t tiles_x, RasterDev rd) {
   grid_dep_wait();
-  uint32_t total = rd.counter[0];
+  // The owner of pair p is the last triangle whose first pair is <= p: first the last block of 256 triangles that starts at or
+  // before p (every stride-th block's start in shared memory, then the rest of the way), then the triangle in it.  With that
+  // and one atomic for the lanes that share a tile a pass over 262k triangles takes 12 us; a search over all the triangles'
+  // prefixes (18 dependent reads) and an atomic a pair took 26, each of the two alone 25.
+  constexpr uint32_t TOP = 2048;
+  __shared__ uint32_t s_top[TOP];
+  const uint32_t total = rd.counter[0], nblk = (ntris + 255u) / 256u, stride = (nblk + TOP - 1u) / TOP, ntop = (nblk + stride - 1u) / stride;
+  if (blockIdx.x * blockDim.x >= total) return;
+  for (uint32_t i = threadIdx.x; i < ntop; i += blockDim.x) s_top[i] = rd.sums[i * stride];
+  __syncthreads();
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = ntris;   // the last triangle whose first pair is <= p: the owner (it has pairs)
+    uint32_t lo = 0, hi = ntop;
     while (hi - lo > 1u) {
-      uint32_t m = (lo + hi) >> 1;
-      if (rd.pre[m] + rd.sums[m >> 8] <= p) lo = m; else hi = m;
+      const uint32_t m = (lo + hi) >> 1;
+      if (s_top[m] <= p) lo = m; else hi = m;
+    }
+    hi = min((lo + 1u) * stride, nblk);
+    lo *= stride;
+    while (hi - lo > 1u) {
+      const uint32_t m = (lo + hi) >> 1;
+      if (rd.sums[m] <= p) lo = m; else hi = m;
+    }
+    const uint32_t in = p - rd.sums[lo];
+    hi = min((lo + 1u) * 256u, ntris);
+    lo *= 256u;
+    while (hi - lo > 1u) {
+      const uint32_t m = (lo + hi) >> 1;
+      if (rd.pre[m] <= in) lo = m; else hi = m;
     }
     uint32_t first = rd.pre[lo] + rd.sums[lo >> 8], nt = rd.ntile[lo];
     if (first + nt > rd.list_cap) {
@@ -193,10 +215,14 @@ __global__ void __launch_bounds__(256) k_rs_bin(uint32_t ntris, uint32_t tiles_x
     uint32_t tx0 = (bx & 0xffffu) / RT, tw = (bx >> 16) / RT - tx0 + 1u, ty0 = (by & 0xffffu) / RT;
     uint32_t i = p - first;
     uint32_t tile = (ty0 + i / tw) * tiles_x + tx0 + i % tw;
+    // neighbouring pairs often share a tile: one atomic for the lanes that do
+    const uint32_t lane = threadIdx.x & 31u, grp = __match_any_sync(__activemask(), tile), rank = __popc(grp & ((1u << lane) - 1u));
     if (!FILL) {
-      atomicAdd(&rd.tile_cnt[tile], 1u);
+      if (rank == 0u) atomicAdd(&rd.tile_cnt[tile], (uint32_t)__popc(grp));
     } else {
-      uint32_t slot = atomicAdd(&rd.tile_fill[tile], 1u);
+      uint32_t slot = 0;
+      if (rank == 0u) slot = atomicAdd(&rd.tile_fill[tile], (uint32_t)__popc(grp));
+      slot = __shfl_sync(grp, slot, __ffs(grp) - 1) + rank;
       rd.list[rd.tile_cnt[tile] + slot] = lo;
     }
   }
@@ -251,79 +277,133 @@ __device__ __forceinline__ uint32_t block_min_256(uint32_t x, uint32_t *ws) {
   return r;
 }
 
-// One block per tile: the tile's list, then the overflow list, in chunks of 256 sorted by depth bound (largest
-// first), fragments of alpha-masked materials whose alpha falls below the cutoff left out; then the winner's depth,
-// normal and style tag
+// One block per tile: the tile's list, then the overflow list, in chunks of 256 triangles, each triangle's record and its box
+// clipped to the tile in shared memory.  A chunk's large triangles (more than RS_SMALL pixels of the tile) are walked by every
+// pixel's thread, front to back by depth bound as above.  The small ones, most of a detailed scene, are dealt out: their
+// (triangle, pixel) pairs go 256 at a time to the block's threads, the keys meeting in shared memory by atomic maxima (the
+// order of which does not matter).  With every triangle walked by all 256 threads a triangle of nine pixels cost as much as
+// one that fills the tile, and the whole chunk was sorted.  Bound by issue (81 % active, some 120 instructions a row of ray
+// tests): 262k triangles at 1920 x 1080 281 -> 203 us, at 1280 x 720 287 -> 135, 26k at 640 x 360 51 -> 27 (dealt over a warp
+// instead of the block: 242, 143, 36).  Taking a long list or a chunk's small ones in bands of depth bound, nearest first,
+// pruned nothing (203 and 222 us).  Fragments of alpha-masked materials whose alpha falls below the cutoff are left out;
+// then the winner's depth, normal and style tag.
+constexpr uint32_t RS_SMALL = 96;   // 48: 211 us on the first of these, 144: 215
 __global__ void __launch_bounds__(256) k_rs_tiles(SceneDev s, const float *__restrict__ F, uint32_t W, uint32_t H,
                                                   uint32_t tiles_x, RasterDev rd, float *depth, uint2 *normal,
                                                   uint8_t *tag) {
   grid_dep_wait();
   __shared__ float4 sa[256], se1[256], se2[256];
-  __shared__ uint32_t skey[256], sval[256];
-  __shared__ uint32_t ws[8];
-  uint32_t tile = blockIdx.x;
-  uint32_t x = (tile % tiles_x) * RT + (threadIdx.x % RT), y = (tile / tiles_x) * RT + (threadIdx.x / RT);
-  bool inside = x < W && y < H;
-  f3 eye = mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2]);
+  __shared__ uint32_t sval[256], s_large[256], s_order[256], s_first[256], s_geo[256];
+  __shared__ float sdx[256], sdy[256], sdz[256];
+  __shared__ unsigned long long s_best[256];
+  __shared__ uint32_t ws[8], s_nlarge;
+  const uint32_t tile = blockIdx.x;
+  const uint32_t X0 = (tile % tiles_x) * RT, Y0 = (tile / tiles_x) * RT;
+  const uint32_t x = X0 + threadIdx.x % RT, y = Y0 + threadIdx.x / RT;
+  const bool inside = x < W && y < H;
+  const f3 eye = mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2]);
   f3 dir = mk(0.0f, 0.0f, 0.0f);
   if (inside) dir = world_at(F, (int)x, (int)y, 1.0f) - eye;
+  sdx[threadIdx.x] = dir.x; sdy[threadIdx.x] = dir.y; sdz[threadIdx.x] = dir.z;
+  s_best[threadIdx.x] = 0ull;
   unsigned long long best = 0ull;
   uint32_t my_depth = inside ? 0u : 0x7f800000u;   // depth bits of best (positive floats order as integers)
   for (int pass = 0; pass < 2; pass++) {
-    uint32_t beg = pass == 0 ? rd.tile_cnt[tile] : 0u, end = pass == 0 ? rd.tile_cnt[tile + 1u] : rd.counter[1];
+    const uint32_t beg = pass == 0 ? rd.tile_cnt[tile] : 0u, end = pass == 0 ? rd.tile_cnt[tile + 1u] : rd.counter[1];
     const uint32_t *lst = pass == 0 ? rd.list : rd.over;
     for (uint32_t c0 = beg; c0 < end; c0 += 256u) {
-      uint32_t n = min(256u, end - c0);
-      uint32_t t = 0, kb = 0;   // empty slots sort last (every bound is > 0)
+      const uint32_t n = min(256u, end - c0);
+      if (threadIdx.x == 0) s_nlarge = 0u;
+      uint32_t far = block_min_256(my_depth, ws);   // (also orders the line above and the last chunk's reads before what follows)
+      // this thread's triangle: its record, its pixels in the tile
+      uint32_t area = 0, wdt = 1, org0 = 0;
       if (threadIdx.x < n) {
-        t = lst[c0 + threadIdx.x];
-        kb = __float_as_uint(rd.rec[3u * t].w);
+        const uint32_t t = lst[c0 + threadIdx.x];
+        const float4 a = rd.rec[3u * t], e1 = rd.rec[3u * t + 1u], e2 = rd.rec[3u * t + 2u];
+        sa[threadIdx.x] = a; se1[threadIdx.x] = e1; se2[threadIdx.x] = e2;
+        sval[threadIdx.x] = t;
+        const uint32_t bound = __float_as_uint(a.w);
+        const uint32_t bx = __float_as_uint(e1.w), by = __float_as_uint(e2.w);
+        const uint32_t ax0 = max(bx & 0xffffu, X0), ax1 = min(bx >> 16, min(X0 + RT, W) - 1u);
+        const uint32_t ay0 = max(by & 0xffffu, Y0), ay1 = min(by >> 16, min(Y0 + RT, H) - 1u);
+        if (bound >= far && ax0 <= ax1 && ay0 <= ay1) {   // else no pixel of the tile can take it
+          wdt = ax1 - ax0 + 1u;
+          area = wdt * (ay1 - ay0 + 1u);
+          org0 = (ay0 - Y0) * RT + (ax0 - X0);
+        }
+        if (area > RS_SMALL) s_large[atomicAdd(&s_nlarge, 1u)] = threadIdx.x;
       }
-      skey[threadIdx.x] = kb;
-      sval[threadIdx.x] = t;
       __syncthreads();
-      for (uint32_t k = 2; k <= 256u; k <<= 1) {      // bitonic sort, descending
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          uint32_t i = threadIdx.x, l = i ^ j;
-          if (l > i) {
-            uint32_t a = skey[i], b = skey[l];
-            if ((i & k) == 0 ? a < b : a > b) {
-              skey[i] = b; skey[l] = a;
-              uint32_t v = sval[i]; sval[i] = sval[l]; sval[l] = v;
+      const uint32_t nl = s_nlarge;
+      if (nl != 0u) {
+        if (threadIdx.x < nl) {   // front to back: each finds its place among the others
+          const uint32_t me = s_large[threadIdx.x], kb = __float_as_uint(sa[me].w);
+          uint32_t rank = 0;
+          for (uint32_t j = 0; j < nl; j++) {
+            const uint32_t o = s_large[j], ko = __float_as_uint(sa[o].w);
+            rank += (ko > kb || (ko == kb && o < me)) ? 1u : 0u;
+          }
+          s_order[rank] = me;
+        }
+        __syncthreads();
+        for (uint32_t j = 0; j < nl; j++) {
+          if ((j & 31u) == 31u) far = block_min_256(my_depth, ws);   // every thread reaches it at the same j
+          const uint32_t i = s_order[j];
+          const float4 a = sa[i];
+          const uint32_t bd = __float_as_uint(a.w);
+          if (bd < far) break;                     // no pixel of the tile can take this or a later triangle
+          if (!inside || bd < my_depth) continue;  // this pixel cannot
+          const float4 e1 = se1[i], e2 = se2[i];
+          const uint32_t bx = __float_as_uint(e1.w), by = __float_as_uint(e2.w);
+          if (x < (bx & 0xffffu) || x > (bx >> 16) || y < (by & 0xffffu) || y > (by >> 16)) continue;
+          float uu = 0.0f, vv = 0.0f;
+          const unsigned long long k = pixel_key(F, eye, dir, mk(a.x, a.y, a.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z),
+                                                 sval[i], uu, vv);
+          if (k > best) {
+            if (s.masked) {   // an alpha-masked fragment is discarded (gbuffer.ts:94)
+              f3 off;
+              if (!raster_alpha_ok(s, drawn_tri(s, sval[i], off), (1.0f - uu) - vv, uu, vv)) continue;
             }
+            best = k; my_depth = (uint32_t)(k >> 32);
           }
-          __syncthreads();
         }
+        s_best[threadIdx.x] = best;
+        __syncthreads();
       }
-      if (threadIdx.x < n) {
-        uint32_t u = sval[threadIdx.x];
-        sa[threadIdx.x] = rd.rec[3u * u];
-        se1[threadIdx.x] = rd.rec[3u * u + 1u];
-        se2[threadIdx.x] = rd.rec[3u * u + 2u];
-      }
+      // the small ones' pixels, dealt over the block
+      const uint32_t cells = area <= RS_SMALL ? area : 0u;
+      uint32_t excl;
+      const uint32_t total = block_sum_256(cells, &excl);
+      s_first[threadIdx.x] = excl;
+      // q / wdt for q < 256, wdt <= 16: (q * ceil(4096 / wdt)) >> 12, exact as the excess stays below 256 / 4096 <= 1 / wdt
+      s_geo[threadIdx.x] = org0 | (wdt << 8) | (((4096u + wdt - 1u) / wdt) << 16);
       __syncthreads();
-      uint32_t far = 0;
-      for (uint32_t j = 0; j < n; j++) {
-        if ((j & 31u) == 0) far = block_min_256(my_depth, ws);   // every thread reaches it at the same j
-        float4 a = sa[j];
-        uint32_t bound = __float_as_uint(a.w);
-        if (bound < far) break;                     // no pixel of the tile can take this or a later triangle
-        if (!inside || bound < my_depth) continue;  // this pixel cannot
-        float4 e1 = se1[j], e2 = se2[j];
-        uint32_t bx = __float_as_uint(e1.w), by = __float_as_uint(e2.w);
-        if (x < (bx & 0xffffu) || x > (bx >> 16) || y < (by & 0xffffu) || y > (by >> 16)) continue;
+      for (uint32_t g = threadIdx.x; g < total; g += 256u) {
+        uint32_t i = 0;   // the last triangle whose first pixel is <= g
+#pragma unroll
+        for (uint32_t bit = 128; bit >= 1; bit >>= 1)
+          if (s_first[i + bit] <= g) i += bit;
+        const uint32_t q = g - s_first[i], ge = s_geo[i];
+        const uint32_t wd = (ge >> 8) & 255u, qy = (q * (ge >> 16)) >> 12, pix = (ge & 255u) + qy * RT + (q - qy * wd);
+        const float4 a = sa[i];
+        const uint32_t bd = __float_as_uint(a.w);
+        const unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(&s_best[pix]);
+        if (bd < (uint32_t)(cur >> 32)) continue;   // this pixel cannot take it
+        const float4 e1 = se1[i], e2 = se2[i];
         float uu = 0.0f, vv = 0.0f;
-        unsigned long long k = pixel_key(F, eye, dir, mk(a.x, a.y, a.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z),
-                                         sval[j], uu, vv);
-        if (k > best) {
-          if (s.masked) {   // an alpha-masked fragment is discarded (gbuffer.ts:94)
+        const unsigned long long k = pixel_key(F, eye, mk(sdx[pix], sdy[pix], sdz[pix]), mk(a.x, a.y, a.z), mk(e1.x, e1.y, e1.z),
+                                               mk(e2.x, e2.y, e2.z), sval[i], uu, vv);
+        if (k > cur) {
+          if (s.masked) {
             f3 off;
-            if (!raster_alpha_ok(s, drawn_tri(s, sval[j], off), (1.0f - uu) - vv, uu, vv)) continue;
+            if (!raster_alpha_ok(s, drawn_tri(s, sval[i], off), (1.0f - uu) - vv, uu, vv)) continue;
           }
-          best = k; my_depth = (uint32_t)(k >> 32);
+          atomicMax(&s_best[pix], k);
         }
       }
       __syncthreads();
+      best = s_best[threadIdx.x];
+      if (inside) my_depth = (uint32_t)(best >> 32);
     }
   }
   if (!inside) return;
