@@ -9,14 +9,14 @@
 //    table does not depend on the order of the concurrent inserts (the phase-concurrent deterministic hash table of
 //    Shun & Blelloch, SPAA 2014); compact numbers the keys in slot order with a chained scan instead of an atomic
 //    counter.  The whole solve is then deterministic and equal to the oracle's state word for word;
-//  * registerPixels inserts the 8 keys of each distinct grid cell of a warp once (the lanes in the same cell and LOD
-//    agree on a leader);
+//  * registerPixels inserts the 8 keys of each distinct grid cell of a warp once, eight lanes a cell;
 //  * relocateVox and linkParents run one warp per probe (64 and 8 x 8 threads in the reference); the sums the
 //    reference takes on one thread are still taken by one lane, in the same order;
 //  * indirect dispatches become grid-stride loops over the device-side probe counts;
 //  * the trace is the persistent ray loop of the screen path over the rays of every cascade's live probes.
 
 constexpr uint32_t W_NONE = 0xffffffffu;
+constexpr uint32_t W_CELLS = 4;              // grid cells a gather warp stages at once
 constexpr uint32_t W_COMPACT_SLOTS = 2048;   // hash slots per compact block (8 a thread)
 
 // hash32 (rc.ts:248-250)
@@ -212,34 +212,45 @@ __global__ void __launch_bounds__(256) k_w_register_pixels(RcDev r, WorldDev w) 
   const float *F = r.frame;
   const uint32_t st = max(reinterpret_cast<const uint32_t *>(F)[F_RU + 2], 1u);
   const uint32_t sx = (r.width + st - 1u) / st, sy = (r.height + st - 1u) / st;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  // a warp takes an 8 x 4 tile of the strided pixels (fewer grid cells than a row of 32)
+  const uint32_t wi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u, tw = (sx + 7u) / 8u;
+  const uint32_t ix = (wi % tw) * 8u + (lane & 7u), iy = (wi / tw) * 4u + (lane >> 3);
   int lod = 0;
-  i3 b = mki(0, 0, 0), org0 = mki(0, 0, 0);
+  i3 rel = mki(0, 0, 0);
   bool live = false;
-  if (i < sx * sy) {
-    const int px = (int)((i % sx) * st + st / 2u), py = (int)((i / sx) * st + st / 2u);
+  if (ix < sx && iy < sy) {
+    const int px = (int)(ix * st + st / 2u), py = (int)(iy * st + st / 2u);
     if (px < (int)r.width && py < (int)r.height) {
       const float d = r.depth[(size_t)py * r.width + (size_t)px];
       if (d > 0.0f) {
         const f3 x = world_at(F, px, py, d);
         lod = w_lod_for(F, length3(x - mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2])));
         const float s = w_spacing(F, lod, 0u);
-        b = vfloori(mk(x.x / s, x.y / s, x.z / s));
-        org0 = w_origin(F, s);
-        live = true;
+        const i3 b = vfloori(mk(x.x / s, x.y / s, x.z / s)), o = w_origin(F, s);
+        rel = mki(b.x - o.x, b.y - o.y, b.z - o.z);   // the cell from its grid's origin: keys exist for -1 .. 511
+        live = rel.x >= -1 && rel.y >= -1 && rel.z >= -1 && rel.x <= 511 && rel.y <= 511 && rel.z <= 511;
       }
     }
   }
-  // the lanes whose pixels fall in the same grid cell at the same LOD hold the same 8 keys: one of them inserts them
-  const unsigned long long xy = ((unsigned long long)(uint32_t)b.x << 32) | (uint32_t)b.y;
-  const unsigned long long zl = live ? (((unsigned long long)(uint32_t)b.z << 32) | (uint32_t)lod) : ~0ull;
-  const unsigned grp = __match_any_sync(0xffffffffu, xy) & __match_any_sync(0xffffffffu, zl);
-  if (live && (uint32_t)(__ffs(grp) - 1) == lane) {
-    for (uint32_t k = 0; k < 8u; k++) {
-      const i3 o = w_corner(k);
-      const uint32_t key = w_key_at(mki(b.x + o.x, b.y + o.y, b.z + o.z), org0, lod);
+  // The lanes whose pixels fall in the same grid cell at the same LOD hold the same 8 keys; each distinct cell's keys are
+  // inserted once, by eight lanes at a time, four cells together.  (One lane inserting its cell's eight keys one after the
+  // other, in rows of 32 pixels, took 55 us for 2 M pixels and 30 for 0.9 M; this 36 and 21.)
+  const uint32_t cell = live ? (uint32_t)(rel.x + 1) | ((uint32_t)(rel.y + 1) << 10) | ((uint32_t)(rel.z + 1) << 20) : 0xffffffffu;
+  const unsigned grp = __match_any_sync(0xffffffffu, cell) & __match_any_sync(0xffffffffu, lod);
+  unsigned heads = __ballot_sync(0xffffffffu, live && (uint32_t)(__ffs(grp) - 1) == lane);
+  while (heads != 0u) {
+    unsigned h = heads;
+    for (uint32_t g = 0; g < (lane >> 3); g++) h &= h - 1u;   // this lane's cell: the (lane / 8)-th of those left
+    const int src = h ? __ffs(h) - 1 : 0;
+    const uint32_t c = __shfl_sync(0xffffffffu, cell, src);
+    const int l = __shfl_sync(0xffffffffu, lod, src);
+    if (h) {
+      const i3 o = w_corner(lane & 7u);
+      const uint32_t key = w_key_at(mki((int)(c & 1023u) - 1 + o.x, (int)((c >> 10) & 1023u) - 1 + o.y, (int)(c >> 20) - 1 + o.z),
+                                    mki(0, 0, 0), l);
       if (key != W_NONE && !w_insert(w.keys + w.hash_off[0], w.hash_mask[0], key)) atomicAdd(&r.counts[16], 1u);
     }
+    for (int g = 0; g < 4; g++) heads &= heads - 1u;   // 0 stays 0
   }
 }
 
@@ -714,8 +725,8 @@ __device__ __forceinline__ ToonRecv toon_receive(f3 c0, f3 c1y, f3 c1z, f3 c1x, 
   return out;
 }
 
-// gatherWorld (rc.ts:880-927), one thread per pixel: the eight c0 probes of the pixel's grid cell, weighted
-// trilinearly and by the side of the surface they are on; with relocate 'voxel' the probes voxels hide are skipped
+// gatherWorld (rc.ts:880-927) with relocate 'voxel', one thread per pixel: the eight c0 probes of the pixel's grid cell, weighted
+// trilinearly and by the side of the surface they are on; the probes voxels hide are skipped
 // (retested from two voxels out when every probe is hidden).  Photoreal pixels left black count in words 72-79.
 // TAG (once the G-buffer carries style tags): toon pixels (tag > 0.75) also interpolate the L0/L1 coefficients and
 // go through the receiving operator (the irradiance replaced when the frame's style.y > 0.5), alpha 2 + band + 2 when
@@ -751,7 +762,6 @@ __global__ void __launch_bounds__(256) k_w_gather(RcDev r, VoxDev v, WorldDev w)
     f3 e = mk(0.0f, 0.0f, 0.0f);
     float ws = 0.0f, ww[8];
     uint32_t hidden = 0, qq[8];
-    const bool vrel = w.relocate == 2u;
     const float tagA = TAG ? r.unorm8[r.tag[q]] : 0.0f;
     const bool toon = TAG && tagA > 0.75f;
     f3 l0 = mk(0.0f, 0.0f, 0.0f), ly = l0, lz = l0, lx = l0;   // toon pixels: the L0 / L1 sums
@@ -764,7 +774,7 @@ __global__ void __launch_bounds__(256) k_w_gather(RcDev r, VoxDev v, WorldDev w)
       const f3 dv = pp - x;
       const float side = dot(n, dv) / mx(length3(dv), 1e-5f);
       const float wt = (tw.x * tw.y * tw.z + 1e-4f) * ((side + 1.0f) * (side + 1.0f) * 0.25f + 0.02f);
-      if (vrel && w_seg_occluded(v, xo1, pp, Lo)) { hidden |= 1u << k; ww[k] = wt; qq[k] = qi; continue; }
+      if (w_seg_occluded(v, xo1, pp, Lo)) { hidden |= 1u << k; ww[k] = wt; qq[k] = qi; continue; }
       e = fma3(w_eval_sh<A>(r, qi, y), wt, e);
       ws += wt;
       if (toon) w_sh_l1_add<A>(r, qi, wt, l0, ly, lz, lx);
@@ -801,6 +811,141 @@ __global__ void __launch_bounds__(256) k_w_gather(RcDev r, VoxDev v, WorldDev w)
                                                        (uint32_t)f2h(res.z) | ((uint32_t)f2h(alpha) << 16));
 }
 
+// evalSH (rc.ts:819-829) of a probe's SH as staged (float4 0-6)
+__device__ __forceinline__ f3 w_eval_sh_at(const float4 *__restrict__ sh, const float y[9]) {
+  float v[28];
+#pragma unroll
+  for (int j = 0; j < 7; j++) {
+    const float4 sc = sh[j];
+    v[4 * j] = sc.x; v[4 * j + 1] = sc.y; v[4 * j + 2] = sc.z; v[4 * j + 3] = sc.w;
+  }
+  f3 es = mk(0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int k = 0; k < 9; k++) es = fma3(mk(v[3 * k], v[3 * k + 1], v[3 * k + 2]), y[k], es);
+  return vmax(es, mk(0.0f, 0.0f, 0.0f));
+}
+
+// The L0 and L1 coefficients (basis order 0, y, z, x) of a probe's staged SH, added with weight wt (shL1 + shAdd,
+// rc.ts:831-840)
+__device__ __forceinline__ void w_sh_l1_add_at(const float4 *__restrict__ sh, float wt, f3 &c0, f3 &cy, f3 &cz, f3 &cx) {
+  const float4 a = sh[0], b = sh[1], c = sh[2];
+  c0 = fma3(mk(a.x, a.y, a.z), wt, c0);
+  cy = fma3(mk(a.w, b.x, b.y), wt, cy);
+  cz = fma3(mk(b.z, b.w, c.x), wt, cz);
+  cx = fma3(mk(c.y, c.z, c.w), wt, cx);
+}
+
+// gatherWorld where no probe can be hidden (relocate 'gbuffer' or 'none'): the warp's distinct grid cells are looked up and
+// their probes' positions and SH staged in shared memory once, four cells a round.  The lanes of a warp share a few cells, and
+// each looking up and loading its own eight probes (72 dependent 128-bit loads a pixel) waited on them: 97 -> 74 us for a
+// room at 1280 x 720 in f16.  With voxel relocation the segment tests are most of the work and a warp with more than four
+// cells would run them once a round: staged 375 us against 366 on the colonnade at 1920 x 1080, so that keeps k_w_gather.
+template <int A, bool TAG>
+__global__ void __launch_bounds__(256, 4) k_w_gather_cells(RcDev r, WorldDev w) {
+  grid_dep_wait();
+  // per warp up to four grid cells' eight probes: the stored SH in float4 0-6, the position in 7 (SH words 28-31 are 0)
+  __shared__ float4 s_cell[8][W_CELLS][8][8];
+  __shared__ uint32_t s_probe[8][W_CELLS][8];
+  // a warp takes a 4 x 8 tile of the block's 16 x 16 pixels (neighbouring pixels share probes and segment lengths;
+  // 0.378 ms on the colonnade with 16 x 2 rows, 0.360 with 8 x 4 tiles, 0.354 with 4 x 8, 0.360 with 2 x 16)
+  const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
+  const uint32_t px = blockIdx.x * 16u + (wp & 3u) * 4u + (lane & 3u), py = blockIdx.y * 16u + (wp >> 2) * 8u + (lane >> 2);
+  const bool on = px < r.width && py < r.height;
+  const size_t q = on ? (size_t)py * r.width + px : 0u;
+  const float *F = r.frame;
+  const float d = on ? r.depth[q] : 0.0f;
+  const bool live = d > 0.0f;
+  f3 res = mk(0.0f, 0.0f, 0.0f);
+  float alpha = live ? 1.0f : 0.0f;
+  f3 x = mk(0.0f, 0.0f, 0.0f), n = x, f = x;
+  i3 bb = mki(0, 0, 0), org0 = bb;
+  int lod = 0;
+  float s0 = 1.0f;
+  if (live) {
+    x = world_at(F, (int)px, (int)py, d);
+    const uint2 nn = r.normal[q];
+    n = mk(h2f(nn.x & 0xffffu), h2f(nn.x >> 16), h2f(nn.y & 0xffffu));
+    lod = w_lod_for(F, length3(x - mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2])));
+    s0 = w_spacing(F, lod, 0u);
+    const f3 gp = mk(x.x / s0, x.y / s0, x.z / s0);
+    bb = vfloori(gp);
+    org0 = w_origin(F, s0);
+    f = gp - vi2f(bb);
+  }
+  // The warp's distinct cells, up to four a round (nearly always all of them): lane 8 g + k looks corner k of cell g up, the
+  // lanes load the cells' probes into shared memory together, and each pixel reads its own cell's there.
+  for (unsigned rem = __ballot_sync(0xffffffffu, live); rem != 0u;) {
+    int mine = -1, lead = (int)lane;
+    uint32_t cells = 0;
+#pragma unroll
+    for (uint32_t g = 0; g < W_CELLS; g++) {
+      if (rem == 0u) break;
+      const int src = __ffs(rem) - 1;
+      const int sx = __shfl_sync(0xffffffffu, bb.x, src), sy = __shfl_sync(0xffffffffu, bb.y, src),
+                sz = __shfl_sync(0xffffffffu, bb.z, src), sl = __shfl_sync(0xffffffffu, lod, src);   // by every lane
+      const bool same = sx == bb.x && sy == bb.y && sz == bb.z && sl == lod;
+      const unsigned grp = __ballot_sync(0xffffffffu, same) & rem;
+      if ((grp >> lane) & 1u) mine = (int)g;
+      if ((lane >> 3) == g) lead = src;
+      rem &= ~grp;
+      cells = g + 1u;
+    }
+    {
+      const i3 cb = mki(__shfl_sync(0xffffffffu, bb.x, lead), __shfl_sync(0xffffffffu, bb.y, lead), __shfl_sync(0xffffffffu, bb.z, lead));
+      const i3 co = mki(__shfl_sync(0xffffffffu, org0.x, lead), __shfl_sync(0xffffffffu, org0.y, lead), __shfl_sync(0xffffffffu, org0.z, lead));
+      const int cl = __shfl_sync(0xffffffffu, lod, lead);
+      const i3 o = w_corner(lane & 7u);
+      if ((lane >> 3) < cells)
+        s_probe[wp][lane >> 3][lane & 7u] = w_lookup(w, 0u, w_key_at(mki(cb.x + o.x, cb.y + o.y, cb.z + o.z), co, cl));
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < cells * 64u; i += 32u) {
+      const uint32_t g = i >> 6, k = (i >> 3) & 7u, j = i & 7u, qi = s_probe[wp][g][k];
+      if (qi != W_NONE) s_cell[wp][g][k][j] = j < 7u ? sh_load<A>(r, (size_t)qi * 8u + j) : r.probes[r.c[0].probe_off + qi].pos;
+    }
+    __syncwarp();
+    if (mine >= 0) {
+      const float4 (*cell)[8] = s_cell[wp][mine];
+      const uint32_t *probe = s_probe[wp][mine];
+      float y[9];
+      sh_basis(n, y);
+      f3 e = mk(0.0f, 0.0f, 0.0f);
+      float ws = 0.0f;
+      const float tagA = TAG ? r.unorm8[r.tag[q]] : 0.0f;
+      const bool toon = TAG && tagA > 0.75f;
+      f3 l0 = mk(0.0f, 0.0f, 0.0f), ly = l0, lz = l0, lx = l0;   // toon pixels: the L0 / L1 sums
+      for (uint32_t k = 0; k < 8u; k++) {
+        const i3 o = w_corner(k);
+        if (probe[k] == W_NONE) continue;
+        const f3 tw = mk(o.x == 1 ? f.x : 1.0f - f.x, o.y == 1 ? f.y : 1.0f - f.y, o.z == 1 ? f.z : 1.0f - f.z);
+        const f3 pp = ld3(cell[k][7]);
+        const f3 dv = pp - x;
+        const float side = dot(n, dv) / mx(length3(dv), 1e-5f);
+        const float wt = (tw.x * tw.y * tw.z + 1e-4f) * ((side + 1.0f) * (side + 1.0f) * 0.25f + 0.02f);
+        e = fma3(w_eval_sh_at(cell[k], y), wt, e);
+        ws += wt;
+        if (toon) w_sh_l1_add_at(cell[k], wt, l0, ly, lz, lx);
+      }
+      if (ws > 0.0f) res = e / ws;
+      if (TAG) {
+        if (toon && ws > 0.0f) {
+          const float iw = 1.0f / ws;
+          const ToonRecv tr = toon_receive(l0 * iw, ly * iw, lz * iw, lx * iw, n, F[F_STYLE + 2]);
+          if (F[F_STYLE + 1] > 0.5f) res = tr.e;
+          alpha = 2.0f + tr.band + (tr.contrast >= 0.1f ? 2.0f : 0.0f);
+        } else if (toon || tagA > 0.25f) {
+          alpha = 2.0f;
+        }
+      }
+    }
+    if (rem != 0u) __syncwarp();   // the next round's cells overwrite these
+  }
+  if (!on) return;
+  if ((A == GI_ATLAS_F32 || r.f32_out) && !r.irr_f16) reinterpret_cast<float4 *>(r.irr)[q] = make_float4(res.x, res.y, res.z, alpha);
+  else reinterpret_cast<uint2 *>(r.irr)[q] = make_uint2((uint32_t)f2h(res.x) | ((uint32_t)f2h(res.y) << 16),
+                                                       (uint32_t)f2h(res.z) | ((uint32_t)f2h(alpha) << 16));
+}
+
 // One world-probe solve (Rc.encode, rc.ts:1180-1221): giBuild (clear .. linkParents), giTrace (the bounce volume, the
 // trace), giMerge (mergeWorld N-1 .. 0, projectSH), giGather
 template <int A>
@@ -815,7 +960,7 @@ static cudaError_t launch_world(const RcDev &r, const VoxDev &v, const WorldDev 
   if (ev) cudaEventRecord(ev[0], st);
   const uint32_t clear_n = max(max(w.hash_total, w.look_total), max(w.hist_h, 96u));
   GI_TRY(gi_launch(k_w_clear, blocks(clear_n), 256, st, r, w));
-  GI_TRY(gi_launch(k_w_register_pixels, (r.width * r.height + 255u) / 256u, 256, st, r, w));
+  GI_TRY(gi_launch(k_w_register_pixels, (((r.width + 7u) / 8u) * ((r.height + 3u) / 4u) + 7u) / 8u, 256, st, r, w));
   // blocks of each task (compact: one per 2048 slots; the others grid-stride over the probes' warps or threads)
   auto nb_compact = [&](uint32_t c) { return (w.hash_mask[c] + W_COMPACT_SLOTS) / W_COMPACT_SLOTS; };
   auto nb_warps = [&](uint32_t c) { return blocks((uint64_t)w.cap[c] * 32u); };
@@ -848,8 +993,14 @@ static cudaError_t launch_world(const RcDev &r, const VoxDev &v, const WorldDev 
     GI_TRY(gi_launch(k_w_merge<A>, blocks((uint64_t)w.cap[c] << r.c[c].dirs_log2), 256, st, r, w, (uint32_t)c));
   GI_TRY(gi_launch(k_w_project_sh<A>, blocks(w.cap[0]), 256, st, r, w));
   if (ev) cudaEventRecord(ev[3], st);
-  if (r.tag_any) GI_TRY(gi_launch(k_w_gather<A, true>, dim3((r.width + 15u) / 16u, (r.height + 15u) / 16u), 256, st, r, v, w));
-  else GI_TRY(gi_launch(k_w_gather<A, false>, dim3((r.width + 15u) / 16u, (r.height + 15u) / 16u), 256, st, r, v, w));
+  const dim3 gg((r.width + 15u) / 16u, (r.height + 15u) / 16u);
+  if (w.relocate != 2u) {
+    if (r.tag_any) GI_TRY(gi_launch(k_w_gather_cells<A, true>, gg, 256, st, r, w));
+    else GI_TRY(gi_launch(k_w_gather_cells<A, false>, gg, 256, st, r, w));
+  } else {
+    if (r.tag_any) GI_TRY(gi_launch(k_w_gather<A, true>, gg, 256, st, r, v, w));
+    else GI_TRY(gi_launch(k_w_gather<A, false>, gg, 256, st, r, v, w));
+  }
   if (ev) cudaEventRecord(ev[4], st);
   return cudaGetLastError();
 }
