@@ -195,132 +195,141 @@ __device__ __forceinline__ f3 shade_voxel(const VoxDev &v, const float *__restri
 
 struct TraceOut { f3 rad; float T; uint32_t lvl, ptr, bit, tin, steps; };
 
-// traceVox (voxel.ts:121-202) as its set-up and one iteration of its loop; the f32 operations and their order are the
-// reference's.  The box of each level and 1 / d come from tables (VoxDev.box_lo/box_hi, RcDev.idirs) holding the
-// same numbers.
-struct Dda {
-  f3 o, d, inv, lo, tMax, tDelta, sp;
-  i3 c, st;
-  float vs, tEnd, tskip, tIn;
-  uint32_t L, steps;
-};
-enum { DDA_WALK = 0, DDA_MISS = 1, DDA_HIT = 2, DDA_HIT_DROP = 3 };
+// traceVox (voxel.ts:121-202) with a configurable step cap: the walk, then the hit's voxShade.  The f32 values that decide
+// anything (exit times, entered cells) come from the reference's operations in its order; the walk's form is its own:
+//  * an empty brick's exits depend only on the brick (absolute plane coordinates), so a run of empty bricks carries the
+//    brick's far planes and pointer index; the cell, its division and its exits, which the reference recomputes at every
+//    jump, are computed once, on entering a brick that holds voxels;
+//  * inside a brick the cell is its 9-bit index plus, per axis, the cells left before the far face (3 bits and a guard
+//    each, from bit 16): a step is one addition, leaving the brick sets a guard, and only then is the next brick's pointer
+//    read.  The bricks left before the clipmap's edge are packed likewise in `rem`;
+//  * the whole warp calls it (lanes without a ray pass live = false), and its lanes meet again before the hits are shaded:
+//    left to themselves they shaded in 2.6 groups of 4.5 lanes a warp.
+// Bound by instruction issue at half-empty warps (12.6 steps a warp for 6 a ray; 131 M warp instructions against 147 M on
+// the colonnade, 69 % issue-active at 24 warps an SM).  Traces, before and after: colonnade 165 -> 163 us, its world probes
+// 94 -> 85, leak room 39 -> 32, textured room 43 -> 36, served 640 x 360 48 -> 40, bounce volumes 62 -> 53 and 88 -> 72.
+// Where the descriptors lie in global memory the walk gains nothing (batch of 8: 324 -> 340).  Nested loops for the two
+// kinds of step took 424 us on the colonnade, 64 registers by recomputing 172, dropping the meeting point 173.
+// inv_pre: the direction's 1 / d with tiny components clamped, tabulated with the directions (the same IEEE quotients), or
+// null to divide here.
+__device__ __forceinline__ bool brick_empty(uint32_t ptr) { return ptr >= GI_MARK && ptr != GI_DROP; }
 
-// what the walk needs besides its position: the level's voxel size and box, the step signs and the cell increments
-__device__ __forceinline__ void dda_derived(const VoxDev &v, Dda &s) {
-  s.vs = vox_size(v, s.L);
-  s.lo = mk(v.box_lo[s.L][0], v.box_lo[s.L][1], v.box_lo[s.L][2]);
-  const f3 dd = mk(fabsf(s.d.x) < 1e-9f ? 1e-9f : s.d.x, fabsf(s.d.y) < 1e-9f ? 1e-9f : s.d.y,
-                   fabsf(s.d.z) < 1e-9f ? 1e-9f : s.d.z);
-  s.st = mki(dd.x > 0.0f ? 1 : -1, dd.y > 0.0f ? 1 : -1, dd.z > 0.0f ? 1 : -1);
-  s.sp = mk(s.st.x > 0 ? 1.0f : 0.0f, s.st.y > 0 ? 1.0f : 0.0f, s.st.z > 0 ? 1.0f : 0.0f);
-  s.tDelta = vabs(s.inv * s.vs);
-}
-
-// traceVox's set-up (voxel.ts:122-138): false when the interval misses the level's box (T = 1, no step taken).
-// inv_pre: the direction's 1 / d with tiny components clamped, tabulated with the directions (the same IEEE
-// quotients), or null to divide here.
-__device__ __forceinline__ bool dda_begin(const VoxDev &v, f3 o, f3 d, float t0, float t1, float tskip, uint32_t L,
-                                          const float4 *inv_pre, Dda &s) {
-  s.o = o; s.d = d; s.L = L; s.steps = 0; s.tskip = tskip;
-  if (inv_pre) {
-    const float4 q = __ldg(inv_pre);
-    s.inv = mk(q.x, q.y, q.z);
-  } else {
-    const f3 dd = mk(fabsf(d.x) < 1e-9f ? 1e-9f : d.x, fabsf(d.y) < 1e-9f ? 1e-9f : d.y, fabsf(d.z) < 1e-9f ? 1e-9f : d.z);
-    s.inv = mk(1.0f / dd.x, 1.0f / dd.y, 1.0f / dd.z);
-  }
-  dda_derived(v, s);
-  const f3 hi = mk(v.box_hi[L][0], v.box_hi[L][1], v.box_hi[L][2]);
-  const f3 ta = (s.lo - o) * s.inv, tb = (hi - o) * s.inv;
-  const f3 tn = vmin(ta, tb), tf = vmax(ta, tb);
-  const float t = mx(mx(mx(tn.x, tn.y), tn.z), t0);
-  s.tEnd = mn(mn(mn(tf.x, tf.y), tf.z), t1);
-  if (t >= s.tEnd) return false;
-  const int nVox = (int)v.G * 8;
-  s.c = iclamp3(vfloori(((o + d * t) - s.lo) / s.vs), mki(0, 0, 0), mki(nVox - 1, nVox - 1, nVox - 1));
-  s.tMax = (((vi2f(s.c) + s.sp) * s.vs + s.lo) - o) * s.inv;
-  s.tIn = t;
-  return true;
-}
-
-// One iteration of traceVox's loop (voxel.ts:142-200) under a step cap: DDA_WALK to go on, DDA_MISS when the walk
-// ends empty, DDA_HIT (h = brick, bit, level L) or DDA_HIT_DROP (h = voxAt's brick, bit and coarser level) on the
-// first occupied voxel entered at tIn >= tSkip.  `steps` counts the iterations taken (rc.ts:232-235).
-__device__ __forceinline__ int dda_step(const VoxDev &v, Dda &s, uint32_t cap, uint3 &h) {
-  if (s.steps >= cap) return DDA_MISS;
-  s.steps++;
-  const int G = (int)v.G, nVox = G * 8;
-  const i3 b = mki(s.c.x >> 3, s.c.y >> 3, s.c.z >> 3);
-  const uint32_t ptr = __ldg(&v.ptr[s.L * (uint32_t)(G * G * G) + ((uint32_t)b.z * (uint32_t)G + (uint32_t)b.y) * (uint32_t)G
-                                    + (uint32_t)b.x]);
-  if (ptr == GI_DROP) {
-    // dropped brick: voxel by voxel, each read at the coarser level that holds it
-    const uint3 r = vox_at(v, s.L, s.c);
-    if (r.x != GI_EMPTY && s.tIn >= s.tskip) { h = r; return DDA_HIT_DROP; }
-    const float tx = mn(mn(s.tMax.x, s.tMax.y), s.tMax.z);
-    if (tx >= s.tEnd) return DDA_MISS;
-    s.tIn = tx;
-  } else if (ptr >= GI_MARK) {
-    // empty brick: jump to its exit
-    const f3 bt = (((vi2f(mki(b.x * 8, b.y * 8, b.z * 8)) + s.sp * 8.0f) * s.vs + s.lo) - s.o) * s.inv;
-    const float te = mn(mn(bt.x, bt.y), bt.z);
-    if (te >= s.tEnd) return DDA_MISS;
-    i3 nb = b;
-    if (bt.x <= bt.y && bt.x <= bt.z) nb.x += s.st.x; else if (bt.y <= bt.z) nb.y += s.st.y; else nb.z += s.st.z;
-    if (nb.x < 0 || nb.y < 0 || nb.z < 0 || nb.x >= G || nb.y >= G || nb.z >= G) return DDA_MISS;
-    s.tIn = te;
-    s.c = iclamp3(vfloori(((s.o + s.d * te) - s.lo) / s.vs), mki(nb.x * 8, nb.y * 8, nb.z * 8),
-                  mki(nb.x * 8 + 7, nb.y * 8 + 7, nb.z * 8 + 7));
-    s.tMax = (((vi2f(s.c) + s.sp) * s.vs + s.lo) - s.o) * s.inv;
-    return DDA_WALK;
-  } else {
-    const uint32_t bit = (uint32_t)((s.c.x & 7) + 8 * (s.c.y & 7) + 64 * (s.c.z & 7));
-    const uint32_t occ = __ldg(&v.occ[ptr * 16u + (bit >> 5)]);
-    const float tExit = mn(mn(s.tMax.x, s.tMax.y), s.tMax.z);
-    if ((occ & (1u << (bit & 31u))) != 0u && s.tIn >= s.tskip) { h = make_uint3(ptr, bit, s.L); return DDA_HIT; }
-    if (tExit >= s.tEnd) return DDA_MISS;
-    s.tIn = tExit;
-  }
-  if (s.tMax.x <= s.tMax.y && s.tMax.x <= s.tMax.z) { s.c.x += s.st.x; s.tMax.x += s.tDelta.x; }
-  else if (s.tMax.y <= s.tMax.z) { s.c.y += s.st.y; s.tMax.y += s.tDelta.y; }
-  else { s.c.z += s.st.z; s.tMax.z += s.tDelta.z; }
-  if (s.c.x < 0 || s.c.y < 0 || s.c.z < 0 || s.c.x >= nVox || s.c.y >= nVox || s.c.z >= nVox) return DDA_MISS;
-  return DDA_WALK;
-}
-
-// The shading point of a hit: the voxel's centre and size (for a dropped brick, the coarser voxel that holds the cell)
-__device__ __forceinline__ void dda_hit_voxel(const VoxDev &v, const Dda &s, int kind, uint32_t hl, f3 &pc, float &vsz) {
-  if (kind == DDA_HIT) {
-    pc = s.lo + adds(vi2f(s.c), 0.5f) * s.vs;
-    vsz = s.vs;
-  } else {
-    vsz = vox_size(v, hl);
-    const f3 pcl = s.lo + adds(vi2f(s.c), 0.5f) * s.vs;
-    pc = adds(vfloor(pcl / vsz), 0.5f) * vsz;
-  }
-}
-
-// traceVox (voxel.ts:121-202) with a configurable step cap: the walk, then the hit's voxShade
 template <class BS>
 __device__ __forceinline__ void trace_vox(const VoxDev &v, const float *__restrict__ F, const float *__restrict__ unorm8,
-                                          f3 o, f3 d, float t0, float t1,
+                                          bool live, f3 o, f3 d, float t0, float t1,
                                           float tskip, uint32_t L, uint32_t cap, TraceOut &out, const BS &bs,
                                           const float4 *inv_pre = nullptr) {
+  constexpr uint32_t LEFT_BRICK = 0x08880000u, LEFT_MAP = (1u << 9) | (1u << 19) | (1u << 29);
   out.rad = mk(0.0f, 0.0f, 0.0f); out.T = 1.0f; out.lvl = GI_EMPTY; out.ptr = GI_EMPTY; out.bit = 0; out.tin = 0;
-  out.steps = 0;
-  Dda s;
-  if (!dda_begin(v, o, d, t0, t1, tskip, L, inv_pre, s)) return;
+  const f3 dd = mk(fabsf(d.x) < 1e-9f ? 1e-9f : d.x, fabsf(d.y) < 1e-9f ? 1e-9f : d.y, fabsf(d.z) < 1e-9f ? 1e-9f : d.z);
+  f3 inv;
+  if (inv_pre) {
+    const float4 q = __ldg(inv_pre);
+    inv = mk(q.x, q.y, q.z);
+  } else {
+    inv = mk(1.0f / dd.x, 1.0f / dd.y, 1.0f / dd.z);
+  }
+  const float vs = vox_size(v, L);
+  const f3 lo = mk(v.box_lo[L][0], v.box_lo[L][1], v.box_lo[L][2]);
+  const f3 hi = mk(v.box_hi[L][0], v.box_hi[L][1], v.box_hi[L][2]);
+  const f3 ta = (lo - o) * inv, tb = (hi - o) * inv;
+  const f3 tn = vmin(ta, tb), tf = vmax(ta, tb);
+  float tIn = mx(mx(mx(tn.x, tn.y), tn.z), t0);
+  const float tEnd = mn(mn(mn(tf.x, tf.y), tf.z), t1);
+  const bool walk = live && !(tIn >= tEnd);   // else the interval misses the level's box
+
+  const uint32_t G = v.G;
+  const int n1 = (int)(G * 8u) - 1;
+  const bool px = dd.x > 0.0f, py = dd.y > 0.0f, pz = dd.z > 0.0f;
+  const f3 s8 = mk(px ? 8.0f : -8.0f, py ? 8.0f : -8.0f, pz ? 8.0f : -8.0f);
+  const int sx = px ? 1 : -1, sy = py ? (int)G : -(int)G, sz = pz ? (int)(G * G) : -(int)(G * G);   // pointer strides
+  const f3 tDelta = vabs(inv * vs);
+  // one cell onward along each axis: the 9-bit index by 1, 8 or 64, the axis's cells left by one
+  const uint32_t cx = (px ? 1u : 0u - 1u) - (1u << 16), cy = (py ? 8u : 0u - 8u) - (1u << 20), cz = (pz ? 64u : 0u - 64u) - (1u << 24);
+
+  // the entered cell (as integers in f32, exact), its brick, the brick's far planes in cells
+  i3 ci = iclamp3(vfloori(((o + d * tIn) - lo) / vs), mki(0, 0, 0), mki(n1, n1, n1));
+  f3 c = vi2f(ci);
+  const i3 b = mki(ci.x >> 3, ci.y >> 3, ci.z >> 3);
+  f3 far = vi2f(mki((b.x + (px ? 1 : 0)) * 8, (b.y + (py ? 1 : 0)) * 8, (b.z + (pz ? 1 : 0)) * 8));
+  uint32_t idx = ptr_index(v, L, b);
+  uint32_t rem = (px ? G - 1u - (uint32_t)b.x : (uint32_t)b.x) | ((py ? G - 1u - (uint32_t)b.y : (uint32_t)b.y) << 10)
+               | ((pz ? G - 1u - (uint32_t)b.z : (uint32_t)b.z) << 20);
+  uint32_t ptr = __ldg(&v.ptr[idx]), steps = 0;
+  bool empty = brick_empty(ptr), drop = false, found = false;
+  // exits along the axes: of the cell, or in an empty brick of the brick
+  const f3 sp = mk(px ? 1.0f : 0.0f, py ? 1.0f : 0.0f, pz ? 1.0f : 0.0f);
+  const f3 e0 = empty ? far : c + sp;
+  f3 T = ((e0 * vs + lo) - o) * inv;
+  uint32_t cell = (uint32_t)((ci.x & 7) | ((ci.y & 7) << 3) | ((ci.z & 7) << 6));
+  cell |= ((cell & 7u) ^ (px ? 7u : 0u)) << 16 | (((cell >> 3) & 7u) ^ (py ? 7u : 0u)) << 20 | ((cell >> 6) ^ (pz ? 7u : 0u)) << 24;
   uint3 h = make_uint3(0u, 0u, 0u);
-  int k;
-  while ((k = dda_step(v, s, cap, h)) == DDA_WALK) {}
-  out.steps = s.steps;
-  if (k == DDA_MISS) return;
-  f3 pc;
-  float vsz;
-  dda_hit_voxel(v, s, k, h.z, pc, vsz);
-  out.rad = shade_voxel(v, F, unorm8, h.x, h.y, s.d, s.o + s.d * s.tIn, pc, vsz, bs); out.T = 0.0f;
-  out.lvl = h.z; out.ptr = h.x; out.bit = h.y; out.tin = __float_as_uint(s.tIn);
+  while (walk && steps < cap) {
+    steps++;
+    uint32_t occ = 0;
+    if (ptr < GI_MARK) occ = __ldg(&v.occ[ptr * 16u + ((cell >> 5) & 15u)]);
+    if ((__funnelshift_r(occ, occ, cell) & 1u) != 0u && tIn >= tskip) { h = make_uint3(ptr, cell & 511u, L); found = true; break; }
+    {
+      if (ptr == GI_DROP) {
+        // dropped brick: voxel by voxel, each read at the coarser level that holds it
+        const uint3 r = vox_at(v, L, mki((int)(px ? far.x - 8.0f : far.x) + (int)(cell & 7u),
+                                         (int)(py ? far.y - 8.0f : far.y) + (int)((cell >> 3) & 7u),
+                                         (int)(pz ? far.z - 8.0f : far.z) + (int)((cell >> 6) & 7u)));
+        if (r.x != GI_EMPTY && tIn >= tskip) { h = r; drop = found = true; break; }
+      }
+    }
+    const bool ax = T.x <= T.y && T.x <= T.z, ay = !ax && T.y <= T.z, az = !ax && !ay;
+    const float te = ax ? T.x : (ay ? T.y : T.z);
+    if (te >= tEnd) break;
+    tIn = te;
+    const uint32_t dc = ax ? cx : (ay ? cy : cz);
+    if (ax) T.x += tDelta.x;
+    if (ay) T.y += tDelta.y;
+    if (az) T.z += tDelta.z;
+    cell += dc;
+    if (empty || (cell & LEFT_BRICK)) {   // into the next brick, at its near face
+      cell -= dc << 3;
+      rem -= ax ? 1u : (ay ? 1u << 10 : 1u << 20);
+      if (rem & LEFT_MAP) break;
+      idx += (uint32_t)(ax ? sx : (ay ? sy : sz));
+      ptr = __ldg(&v.ptr[idx]);
+      if (ax) far.x += s8.x;
+      if (ay) far.y += s8.y;
+      if (az) far.z += s8.z;
+      const bool was = empty;
+      empty = brick_empty(ptr);
+      f3 e = far;
+      if (was && !empty) {
+        // the entered cell: floor by an addition rounded down (exact for |q| < 2^22), clamped to the entered brick
+        const f3 q = ((o + d * tIn) - lo) / vs;
+        const f3 near = mk(px ? far.x - 8.0f : far.x, py ? far.y - 8.0f : far.y, pz ? far.z - 8.0f : far.z);
+        c = mk(fminf(fmaxf(__fadd_rd(q.x, 12582912.0f) - 12582912.0f, near.x), near.x + 7.0f),
+               fminf(fmaxf(__fadd_rd(q.y, 12582912.0f) - 12582912.0f, near.y), near.y + 7.0f),
+               fminf(fmaxf(__fadd_rd(q.z, 12582912.0f) - 12582912.0f, near.z), near.z + 7.0f));
+        const uint32_t lx = (uint32_t)__float_as_int(c.x + 8388608.0f) & 7u, ly = (uint32_t)__float_as_int(c.y + 8388608.0f) & 7u,
+                       lz = (uint32_t)__float_as_int(c.z + 8388608.0f) & 7u;
+        cell = (lx | (ly << 3) | (lz << 6)) | ((px ? lx ^ 7u : lx) << 16) | ((py ? ly ^ 7u : ly) << 20) | ((pz ? lz ^ 7u : lz) << 24);
+        e = c + sp;
+      }
+      if (was || empty) T = ((e * vs + lo) - o) * inv;
+    }
+  }
+  out.steps = steps;
+  __syncwarp();
+  if (found) {
+    // the shading point: the voxel's centre and size (for a dropped brick, the coarser voxel that holds the cell)
+    c = mk((px ? far.x - 8.0f : far.x) + (float)(cell & 7u), (py ? far.y - 8.0f : far.y) + (float)((cell >> 3) & 7u),
+           (pz ? far.z - 8.0f : far.z) + (float)((cell >> 6) & 7u));
+    f3 pc = lo + adds(c, 0.5f) * vs;
+    float vsz = vs;
+    if (drop) {
+      vsz = vox_size(v, h.z);
+      pc = adds(vfloor(pc / vsz), 0.5f) * vsz;
+    }
+    out.rad = shade_voxel(v, F, unorm8, h.x, h.y, d, o + d * tIn, pc, vsz, bs); out.T = 0.0f;
+    out.lvl = h.z; out.ptr = h.x; out.bit = h.y; out.tin = __float_as_uint(tIn);
+  }
+  __syncwarp();
 }
 
 // ---- the dynamic layer's read (dynlayer.ts:71-162) ------------------------------------------------------------------
@@ -492,16 +501,14 @@ __device__ __forceinline__ uint32_t dir_tile(const CascDev &L, uint32_t k) {
 }
 
 // trace (rc.ts:600-622) -> traceWorld (rc.ts:216-245) of the ray at position j of the trace order (cascade c): writes
-// its atlas element (and the debug copies); true when its probe is valid and the ray was marched.
+// its atlas element (and the debug copies) when live; true when its probe is valid and the ray was marched.  The whole
+// warp calls it (trace_vox); lanes without a ray pass live = false and the position of any ray.
 template <int A, bool DYN = false>
-__device__ __forceinline__ bool trace_ray(const RcDev &r, const VoxDev &v, uint32_t j, uint32_t c, TraceOut &out,
+__device__ __forceinline__ bool trace_ray(const RcDev &r, const VoxDev &v, uint32_t j, uint32_t c, bool live, TraceOut &out,
                                           bool probe_major) {
   typedef typename Atlas<A>::T T;
   T *rad = reinterpret_cast<T *>(r.rad);
   const float *F = r.frame;
-  out.rad = mk(0.0f, 0.0f, 0.0f); out.T = 1.0f; out.lvl = GI_EMPTY; out.ptr = GI_EMPTY; out.bit = 0; out.tin = 0;
-  out.steps = 0;
-  bool traced = false;
   const CascDev &L = r.c[c];
   uint32_t t = j - L.ray_off, pi, di;
   if (probe_major) {                  // probe-major: a probe's rays together; a warp's on neighbouring directions
@@ -514,23 +521,23 @@ __device__ __forceinline__ bool trace_ray(const RcDev &r, const VoxDev &v, uint3
   }
   uint32_t i = L.ray_off + (pi << L.dirs_log2) + di;   // the ray's atlas element
   ProbeDev pr = r.probes[L.probe_off + pi];
-  if (pr.pos.w > 0.0f) {
-    float4 dv = r.dirs[L.dir_off + di];   // dirOf(di, res), tabulated
-    f3 dir = mk(dv.x, dv.y, dv.z);
-    float s0 = pr.pos.w;
-    float t0 = L.b0 * s0, t1 = L.b1 * s0;
-    f3 po = ld3(pr.pos), pn = ld3(pr.nrm);
-    uint32_t Lv = vox_level_for(v, r.plevel[L.probe_off + pi], po + dir * t1);
-    float vs = vox_size(v, Lv);
-    const f3 ooff = po + pn * (r.vox_offset * vs);
-    trace_vox(v, F, r.unorm8, ooff, dir, t0, t1, r.vox_skip * vs, Lv, r.dda_cap, out, InjectedBounce{r.bn_inj},
-              r.idirs + L.dir_off + di);
-    if (DYN) dyn_compose(r, v, po, dir, t0, t1, ooff, 3.5449077f / (float)L.res, out);
-    traced = true;
+  const bool traced = live && pr.pos.w > 0.0f;
+  float4 dv = r.dirs[L.dir_off + di];   // dirOf(di, res), tabulated
+  f3 dir = mk(dv.x, dv.y, dv.z);
+  float s0 = pr.pos.w;
+  float t0 = L.b0 * s0, t1 = L.b1 * s0;
+  f3 po = ld3(pr.pos), pn = ld3(pr.nrm);
+  uint32_t Lv = vox_level_for(v, r.plevel[L.probe_off + pi], po + dir * t1);
+  float vs = vox_size(v, Lv);
+  const f3 ooff = po + pn * (r.vox_offset * vs);
+  trace_vox(v, F, r.unorm8, traced, ooff, dir, t0, t1, r.vox_skip * vs, Lv, r.dda_cap, out,
+            InjectedBounce{r.bn_inj}, r.idirs + L.dir_off + di);
+  if (DYN && traced) dyn_compose(r, v, po, dir, t0, t1, ooff, 3.5449077f / (float)L.res, out);
+  if (live) {
+    Atlas<A>::store(rad, i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
+    if (r.hits) r.hits[i] = make_uint4(out.lvl, out.ptr, out.bit, out.tin);
+    if (r.rad_traced) Atlas<A>::store(reinterpret_cast<T *>(r.rad_traced), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
   }
-  Atlas<A>::store(rad, i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
-  if (r.hits) r.hits[i] = make_uint4(out.lvl, out.ptr, out.bit, out.tin);
-  if (r.rad_traced) Atlas<A>::store(reinterpret_cast<T *>(r.rad_traced), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
   return traced;
 }
 
@@ -610,10 +617,10 @@ __global__ void __launch_bounds__(256) k_trace(RcDev r, VoxDev v, uint32_t *ray_
     bool live = j < r.rays_total;
     if (SORT && live) j = r.rperm[j];     // the atlas element at that position
     else if (live) j = r.rays_total - 1u - j;   // the top cascade first: the queue ends on the shortest walks
-    uint32_t c = live ? casc_of_ray(r, j) : 0u;
+    if (!live) j = 0u;
+    uint32_t c = casc_of_ray(r, j);
     TraceOut out;
-    out.steps = 0;
-    bool traced = live && trace_ray<A, DYN>(r, v, j, c, out, SORT || r.trace_order == 0u);
+    bool traced = trace_ray<A, DYN>(r, v, j, c, live, out, SORT || r.trace_order == 0u);
     if (SORT && live) r.rsteps[j] = (uint8_t)rsort_key(traced ? out.steps : 0u, traced && out.T < 0.5f);
     if (r.stats) {
       // per-cascade counters (rc.ts:232-235); flush when the lane's cascade changes
@@ -1011,22 +1018,26 @@ __global__ void __launch_bounds__(256) k_bn_classify(BounceDev b, VoxDev v, cons
 }
 
 // bnTrace (bounce.ts:156-167): the ray in segments [b_k, b_k+1] cells (b_k = (4^k - 1) / 3) on level k's voxels;
-// rgb and the distance to the hit (sky and 1e9 past the last level)
-__device__ float4 bn_trace(const VoxDev &v, const float *__restrict__ F, const float *__restrict__ unorm8,
-                           const BounceDev &b, const uint2 *prev, f3 o, f3 d, float tmax) {
+// rgb and the distance to the hit (sky and 1e9 past the last level).  The whole warp calls it (trace_vox).
+__device__ __forceinline__ float4 bn_trace(const VoxDev &v, const float *__restrict__ F, const float *__restrict__ unorm8,
+                                           const BounceDev &b, const uint2 *prev, bool live, f3 o, f3 d, float tmax) {
+  float4 res = make_float4(F[F_SKY], F[F_SKY + 1], F[F_SKY + 2], 1e9f);
   float b0 = 0.0f;
-  for (uint32_t k = 0; k < v.levels && b0 * b.cell < tmax; k++) {
+  for (uint32_t k = 0; k < v.levels; k++) {
+    live = live && b0 * b.cell < tmax;
+    if (!__any_sync(0xffffffffu, live)) break;
     const float b1 = b0 * 4.0f + 1.0f;
     const uint32_t L = vox_level_for(v, k, o + (d * b1) * b.cell);
     TraceOut r;
-    trace_vox(v, F, unorm8, o, d, b0 * b.cell, mn(b1 * b.cell, tmax), 0.0f, L, BN_DDA_CAP, r, VolumeBounce{&b, prev});
+    trace_vox(v, F, unorm8, live, o, d, b0 * b.cell, mn(b1 * b.cell, tmax), 0.0f, L, BN_DDA_CAP, r, VolumeBounce{&b, prev});
     if (r.T < 0.5f) {
       const f3 entry = o + d * __uint_as_float(r.tin);
-      return make_float4(r.rad.x, r.rad.y, r.rad.z, dot(entry - o, d));
+      res = make_float4(r.rad.x, r.rad.y, r.rad.z, dot(entry - o, d));
+      live = false;
     }
     b0 = b1;
   }
-  return make_float4(F[F_SKY], F[F_SKY + 1], F[F_SKY + 2], 1e9f);
+  return res;
 }
 
 // bnUpdate (bounce.ts:172-208) in two launches.  k_bn_rays: one thread per ray of a listed probe, the probe's rays
@@ -1047,26 +1058,26 @@ __global__ void __launch_bounds__(256) k_bn_rays(BounceDev b, VoxDev v, RcDev r)
   const uint32_t per = b.rays + 6u, total = b.list[0] * per;
   const uint2 *prev = b.vol[b.list[2] ^ 1u];
   const i3 o = bn_origin_now(b, F);
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t w = blockIdx.x * blockDim.x + (threadIdx.x - lane); w < total; w += gridDim.x * blockDim.x) {
+    const bool live = w + lane < total;
+    const uint32_t t = live ? w + lane : w;
     const uint32_t slot = t / per, k = t - slot * per;
     const uint32_t i = b.list[4u + slot];
     const i3 c = mki((int)(i % b.dx), (int)((i / b.dx) % b.dy), (int)(i / (b.dx * b.dy)));
     const f3 p = vi2f(mki(o.x + c.x, o.y + c.y, o.z + c.z)) * b.cell;
-    float4 res;
-    if (k < b.rays) {
-      const float4 dv = b.dirs[k];
-      res = bn_trace(v, F, unorm8, b, prev, p, mk(dv.x, dv.y, dv.z), 1e9f);
-      if (DYN) {
-        const float4 dl = trace_dyn(r, v, p, mk(dv.x, dv.y, dv.z), 0.0f, mn(res.w, 1e4f),
-                                    sqrtf((4.0f * GI_PI) / (float)b.rays));
-        const float s = 1.0f - dl.w;
-        res = make_float4(dl.x + s * res.x, dl.y + s * res.y, dl.z + s * res.z, res.w);
-      }
-    } else {
-      res = make_float4(0.0f, 0.0f, 0.0f,
-                        mx(mn(bn_trace(v, F, unorm8, b, prev, p, bn_axis_vec(k - b.rays), 1.5f * b.cell).w, 1.5f * b.cell), 1e-3f));
+    const bool axis = k >= b.rays;
+    const float4 dv = b.dirs[axis ? 0u : k];
+    const f3 d = axis ? bn_axis_vec(k - b.rays) : mk(dv.x, dv.y, dv.z);
+    float4 res = bn_trace(v, F, unorm8, b, prev, live, p, d, axis ? 1.5f * b.cell : 1e9f);
+    if (axis) {
+      res = make_float4(0.0f, 0.0f, 0.0f, mx(mn(res.w, 1.5f * b.cell), 1e-3f));
+    } else if (DYN) {
+      const float4 dl = trace_dyn(r, v, p, d, 0.0f, mn(res.w, 1e4f), sqrtf((4.0f * GI_PI) / (float)b.rays));
+      const float s = 1.0f - dl.w;
+      res = make_float4(dl.x + s * res.x, dl.y + s * res.y, dl.z + s * res.z, res.w);
     }
-    b.ray_out[t] = res;
+    if (live) b.ray_out[t] = res;
   }
 }
 __global__ void __launch_bounds__(256) k_bn_sum(BounceDev b) {
@@ -1271,11 +1282,11 @@ __global__ void __launch_bounds__(256) k_trace_batch(BatchDev B) {
     if (base >= total) break;
     const uint32_t s = batch_owner(B.ray_pre, B.n, base);
     const RcDev &r = B.rc[s];
-    const uint32_t j = base - B.ray_pre[s] + lane;
-    if (j < r.rays_total) {
-      TraceOut out;
-      trace_ray<A>(r, B.vox[s], j, casc_of_ray(r, j), out, r.trace_order != 1u);
-    }
+    uint32_t j = base - B.ray_pre[s] + lane;
+    const bool live = j < r.rays_total;
+    if (!live) j = 0u;
+    TraceOut out;
+    trace_ray<A>(r, B.vox[s], j, casc_of_ray(r, j), live, out, r.trace_order != 1u);
   }
 }
 

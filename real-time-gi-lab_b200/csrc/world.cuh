@@ -465,32 +465,30 @@ __global__ void __launch_bounds__(256) k_w_build(RcDev r, VoxDev v, WorldDev w, 
   else w_task(r, v, w, tb, cb, blockIdx.x - na, nb);
 }
 
-// trace (rc.ts:600-622) of ray (pi, di) of a world probe of cascade c into atlas element i
+// trace (rc.ts:600-622) of ray (pi, di) of a world probe of cascade c into atlas element i when live.  The whole warp
+// calls it (trace_vox); lanes without a ray pass live = false and any live probe's ray.
 template <int A, bool DYN>
 __device__ __forceinline__ bool w_trace_ray(const RcDev &r, const VoxDev &v, uint32_t c, uint32_t pi, uint32_t di,
-                                            size_t i, TraceOut &out) {
+                                            size_t i, bool live, TraceOut &out) {
   typedef typename Atlas<A>::T T;
-  out.rad = mk(0.0f, 0.0f, 0.0f); out.T = 1.0f; out.lvl = GI_EMPTY; out.ptr = GI_EMPTY; out.bit = 0; out.tin = 0;
-  out.steps = 0;
-  bool traced = false;
   const CascDev &L = r.c[c];
   const ProbeDev pr = r.probes[L.probe_off + pi];
-  if (pr.pos.w > 0.0f) {
-    const float4 dv = r.dirs[L.dir_off + di];
-    const f3 dir = mk(dv.x, dv.y, dv.z);
-    const float s0 = pr.pos.w, t0 = L.b0 * s0, t1 = L.b1 * s0;
-    const f3 po = ld3(pr.pos), pn = ld3(pr.nrm);
-    const uint32_t Lv = vox_level_for(v, r.plevel[L.probe_off + pi], po + dir * t1);
-    const float vs = vox_size(v, Lv);
-    const f3 ooff = po + pn * (r.vox_offset * vs);
-    trace_vox(v, r.frame, r.unorm8, ooff, dir, t0, t1, r.vox_skip * vs, Lv, r.dda_cap, out, InjectedBounce{r.bn_inj},
-              r.idirs + L.dir_off + di);
-    if (DYN) dyn_compose(r, v, po, dir, t0, t1, ooff, 3.5449077f / (float)L.res, out);
-    traced = true;
+  const bool traced = live && pr.pos.w > 0.0f;
+  const float4 dv = r.dirs[L.dir_off + di];
+  const f3 dir = mk(dv.x, dv.y, dv.z);
+  const float s0 = pr.pos.w, t0 = L.b0 * s0, t1 = L.b1 * s0;
+  const f3 po = ld3(pr.pos), pn = ld3(pr.nrm);
+  const uint32_t Lv = vox_level_for(v, r.plevel[L.probe_off + pi], po + dir * t1);
+  const float vs = vox_size(v, Lv);
+  const f3 ooff = po + pn * (r.vox_offset * vs);
+  trace_vox(v, r.frame, r.unorm8, traced, ooff, dir, t0, t1, r.vox_skip * vs, Lv, r.dda_cap, out,
+            InjectedBounce{r.bn_inj}, r.idirs + L.dir_off + di);
+  if (DYN && traced) dyn_compose(r, v, po, dir, t0, t1, ooff, 3.5449077f / (float)L.res, out);
+  if (live) {
+    Atlas<A>::store(reinterpret_cast<T *>(r.rad), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
+    if (r.hits) r.hits[i] = make_uint4(out.lvl, out.ptr, out.bit, out.tin);
+    if (r.rad_traced) Atlas<A>::store(reinterpret_cast<T *>(r.rad_traced), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
   }
-  Atlas<A>::store(reinterpret_cast<T *>(r.rad), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
-  if (r.hits) r.hits[i] = make_uint4(out.lvl, out.ptr, out.bit, out.tin);
-  if (r.rad_traced) Atlas<A>::store(reinterpret_cast<T *>(r.rad_traced), i, make_float4(out.rad.x, out.rad.y, out.rad.z, out.T));
   return traced;
 }
 
@@ -516,13 +514,10 @@ __global__ void __launch_bounds__(256) k_w_trace(RcDev r, VoxDev v, WorldDev w, 
       for (uint32_t q = 1; q < r.cascades; q++)
         if (j >= s_first[q]) c = q;
       TraceOut out;
-      out.steps = 0;
-      bool traced = false;
-      if (live) {
-        const CascDev &L = r.c[c];
-        const uint32_t t = j - s_first[c];
-        traced = w_trace_ray<A, DYN>(r, v, c, t >> L.dirs_log2, t & ((1u << L.dirs_log2) - 1u), (size_t)L.rad_off + t, out);
-      }
+      const CascDev &L = r.c[c];
+      const uint32_t t = j - s_first[c];
+      const bool traced = w_trace_ray<A, DYN>(r, v, c, t >> L.dirs_log2, t & ((1u << L.dirs_log2) - 1u),
+                                              (size_t)L.rad_off + t, live, out);
       if (r.stats && live && traced) {   // per-cascade counters (rc.ts:232-235)
         if (c != cur_c && cur_c != 0xffffffffu) {
           atomicAdd(&r.counts[24 + cur_c], traces_acc); atomicAdd(&r.counts[32 + cur_c], steps_acc);
