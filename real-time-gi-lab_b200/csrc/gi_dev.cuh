@@ -471,6 +471,31 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t w, uint32_t r) {
   return pos;
 }
 
+// The brick of voxel ai of the attribute pool: the last b < nb with vpre[b] <= ai.  The whole warp calls it with consecutive
+// ai0 + lane; the first lane's brick by a 32-way search (lane k reads the prefix at lo + span (k + 1) / 33), then the next 32
+// prefixes in one load, of which a warp's voxels pass a few.  A binary search per voxel was 12 dependent reads: resolveAttr
+// of a colonnade at 1920x1080 29.0 -> 27.9 us, 51.6 -> 49 with a sun's shadow map (bounce at 1600x900), 8.1 -> 7.3 in a room of 256x256.
+__device__ __forceinline__ uint32_t voxel_brick(const uint32_t *__restrict__ vpre, uint32_t nb, uint32_t ai0) {
+  const uint32_t lane = threadIdx.x & 31u, ai = ai0 + lane;
+  uint32_t lo = 0, hi = nb;
+  while (hi - lo > 32u) {
+    const uint32_t span = hi - lo, m = lo + (uint32_t)(((unsigned long long)span * (lane + 1u)) / 33u);
+    const uint32_t k = __popc(__ballot_sync(0xffffffffu, vpre[m] <= ai0));   // the prefixes ascend: the first k probes hold
+    const uint32_t nlo = k ? lo + (uint32_t)(((unsigned long long)span * k) / 33u) : lo;
+    hi = k < 32u ? lo + (uint32_t)(((unsigned long long)span * (k + 1u)) / 33u) : hi;
+    lo = nlo;
+  }
+  lo += __popc(__ballot_sync(0xffffffffu, lo + 1u + lane < hi && vpre[min(lo + 1u + lane, nb - 1u)] <= ai0));
+  uint32_t b = lo;
+  for (uint32_t first = lo + 1u;; first += 32u) {
+    const uint32_t p = first + lane < nb ? vpre[first + lane] : 0xffffffffu;
+    const uint32_t last = __popc(__ballot_sync(0xffffffffu, p <= ai0 + 31u));   // prefixes that some lane has passed
+    for (uint32_t j = 0; j < last; j++) b += __shfl_sync(0xffffffffu, p, (int)j) <= ai ? 1u : 0u;
+    if (last < 32u) break;
+  }
+  return b;
+}
+
 // Warp-aggregated atomicAdd: one atomic per distinct address among the active lanes would need a match; the lists
 // and counters here use one address per call, so the active lanes share it.
 __device__ __forceinline__ uint32_t warp_append(uint32_t *counter, bool want) {

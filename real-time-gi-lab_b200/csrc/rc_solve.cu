@@ -1104,19 +1104,16 @@ __global__ void __launch_bounds__(256) k_bn_sum(BounceDev b) {
 }
 
 // bnInject (bounce.ts:213-246): every occupied voxel stores this frame's volume read on its two sides.  One thread
-// per voxel of the attribute pool (its brick by a binary search of the voxel prefix, as resolveAttr).
+// per voxel of the attribute pool (its brick by voxel_brick, as resolveAttr).
 __global__ void __launch_bounds__(256) k_bn_inject(BounceDev b, VoxDev v) {
   grid_dep_wait();
   const uint2 *cur = b.vol[b.list[2]];
   const uint32_t nb = min(v.hdr[0], v.max_bricks);
   const uint32_t nv = nb ? min(v.vpre[nb], v.max_voxels) : 0u;
-  for (uint32_t ai = blockIdx.x * blockDim.x + threadIdx.x; ai < nv; ai += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = nb;
-    while (hi - lo > 1u) {
-      uint32_t m = (lo + hi) >> 1;
-      if (v.vpre[m] <= ai) lo = m; else hi = m;
-    }
-    const uint32_t ptr = lo;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t ai0 = blockIdx.x * blockDim.x + (threadIdx.x - lane); ai0 < nv; ai0 += gridDim.x * blockDim.x) {
+    const uint32_t ptr = voxel_brick(v.vpre, nb, ai0), ai = ai0 + lane;
+    if (ai >= nv) continue;
     if (v.base[ptr] == GI_EMPTY) continue;
     uint32_t r = ai - v.vpre[ptr], bit = 0;
     const uint4 *o4 = reinterpret_cast<const uint4 *>(v.occ) + ptr * 4u;

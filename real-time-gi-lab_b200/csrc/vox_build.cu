@@ -784,13 +784,10 @@ __global__ void __launch_bounds__(256) k_resolve_attr(VoxDev v, SceneDev s) {
   grid_dep_wait();
   uint32_t nb = min(v.hdr[0], v.max_bricks);
   uint32_t nv = nb ? min(v.vpre[nb], v.max_voxels) : 0u;
-  for (uint32_t ai = blockIdx.x * blockDim.x + threadIdx.x; ai < nv; ai += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = nb;   // the last brick b with vpre[b] <= ai
-    while (hi - lo > 1u) {
-      uint32_t m = (lo + hi) >> 1;
-      if (v.vpre[m] <= ai) lo = m; else hi = m;
-    }
-    uint32_t ptr = lo;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t ai0 = blockIdx.x * blockDim.x + (threadIdx.x - lane); ai0 < nv; ai0 += gridDim.x * blockDim.x) {
+    const uint32_t ptr = voxel_brick(v.vpre, nb, ai0), ai = ai0 + lane;
+    if (ai >= nv) continue;
     if (v.base[ptr] == GI_EMPTY) continue;   // past the voxel pool: no attributes (voxel.ts:586)
     uint32_t r = ai - v.vpre[ptr];
     const uint4 *o4 = reinterpret_cast<const uint4 *>(v.occ) + ptr * 4u;
