@@ -399,12 +399,14 @@ __device__ __forceinline__ float4 trace_dyn(const RcDev &r, const VoxDev &v, f3 
       float f = lf - (float)L0;
       const uint32_t Lw = vox_level_for(v, L0, p);
       if (Lw != L0) { L0 = Lw; f = 0.0f; }
-      uint32_t la, lb;
-      const float4 sa = dyn_read(r, dyn_find(r, v, L0, p, la), la, d);
+      uint32_t la, lb = 0;
+      const bool two = f > 0.0f && L0 + 1u < nl;   // both levels' bricks looked up ahead of either's words
+      const uint32_t fa = dyn_find(r, v, L0, p, la), fb = two ? dyn_find(r, v, L0 + 1u, p, lb) : 0xffffffffu;
+      const float4 sa = dyn_read(r, fa, la, d);
       float aa = sa.w * len / vox_size(v, la);
       f3 ra = mk(sa.x, sa.y, sa.z) * aa;
-      if (f > 0.0f && L0 + 1u < nl) {
-        const float4 sb = dyn_read(r, dyn_find(r, v, L0 + 1u, p, lb), lb, d);
+      if (two) {
+        const float4 sb = dyn_read(r, fb, lb, d);
         const float ab = sb.w * len / vox_size(v, lb);
         const f3 rb = mk(sb.x, sb.y, sb.z) * ab;
         ra = ra * (1.0f - f) + rb * f;   // mix(ra, rb, f)
@@ -602,9 +604,10 @@ __global__ void __launch_bounds__(256) k_rsort_scatter(RcDev r) {
 // Persistent: every warp takes rays from a global counter, 32 x trace_rays at a time, the top cascade's first (its
 // walks are the longest; a queue that ended on them left SMs idle behind its last warps: 0.197 -> 0.170 ms on the
 // colonnade).  SORT: positions go through the walk-length order (rperm) and each ray's key is stored for the next
-// solve.
+// solve.  With the dynamic layer's read (chains of scattered reads) four blocks an SM, 64 registers, instead of the three that
+// the walk's registers alone give: 556 -> 521 us on the colonnade with 64 moving boxes, 247 -> 241 at 1280 x 720.
 template <int A, bool DYN, bool SORT>
-__global__ void __launch_bounds__(256) k_trace(RcDev r, VoxDev v, uint32_t *ray_counter) {
+__global__ void __launch_bounds__(256, DYN ? 4 : 0) k_trace(RcDev r, VoxDev v, uint32_t *ray_counter) {
   grid_dep_wait();
   uint32_t lane = threadIdx.x & 31u;
   uint32_t steps_acc = 0, traces_acc = 0, cap_acc = 0;
