@@ -174,20 +174,23 @@ __global__ void __launch_bounds__(256) k_rs_scan(uint32_t nblk, RasterDev rd) {
 
 // Every (triangle, tile) pair: FILL = false counts the pairs of each tile and lists the triangles that do not fit the
 // list capacity; FILL = true writes each pair's triangle into its tile's range of the list
+constexpr uint32_t RS_SHARE = 4;   // changes of triangle between a warp's pairs
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_rs_bin(uint32_t ntris, uint32_t tiles_x, RasterDev rd) {
   grid_dep_wait();
   // The owner of pair p is the last triangle whose first pair is <= p: first the last block of 256 triangles that starts at or
   // before p (every stride-th block's start in shared memory, then the rest of the way), then the triangle in it.  With that
-  // and one atomic for the lanes that share a tile a pass over 262k triangles takes 12 us; a search over all the triangles'
-  // prefixes (18 dependent reads) and an atomic a pair took 26, each of the two alone 25.
+  // and one atomic for the lanes that share a tile the two passes over 262k triangles at 1280 x 720 take 21 us; a search over all
+  // the triangles' prefixes (18 dependent reads) and an atomic a pair took 60.
   constexpr uint32_t TOP = 2048;
   __shared__ uint32_t s_top[TOP];
   const uint32_t total = rd.counter[0], nblk = (ntris + 255u) / 256u, stride = (nblk + TOP - 1u) / TOP, ntop = (nblk + stride - 1u) / stride;
   if (blockIdx.x * blockDim.x >= total) return;
   for (uint32_t i = threadIdx.x; i < ntop; i += blockDim.x) s_top[i] = rd.sums[i * stride];
   __syncthreads();
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t p0 = blockIdx.x * blockDim.x + (threadIdx.x - lane); p0 < total; p0 += gridDim.x * blockDim.x) {   // whole warps
+    const uint32_t p = min(p0 + lane, total - 1u);
     uint32_t lo = 0, hi = ntop;
     while (hi - lo > 1u) {
       const uint32_t m = (lo + hi) >> 1;
@@ -206,24 +209,28 @@ __global__ void __launch_bounds__(256) k_rs_bin(uint32_t ntris, uint32_t tiles_x
       const uint32_t m = (lo + hi) >> 1;
       if (rd.pre[m] <= in) lo = m; else hi = m;
     }
-    uint32_t first = rd.pre[lo] + rd.sums[lo >> 8], nt = rd.ntile[lo];
-    if (first + nt > rd.list_cap) {
-      if (!FILL && p == first) rd.over[atomicAdd(&rd.counter[1], 1u)] = lo;
-      continue;
-    }
+    const uint32_t first = rd.pre[lo] + rd.sums[lo >> 8], nt = rd.ntile[lo], i = p - first;
+    const bool listed = p0 + lane < total && first + nt <= rd.list_cap;
+    if (!FILL && p0 + lane < total && !listed && i == 0u) rd.over[atomicAdd(&rd.counter[1], 1u)] = lo;
     uint32_t bx = __float_as_uint(rd.rec[3u * lo + 1u].w), by = __float_as_uint(rd.rec[3u * lo + 2u].w);
     uint32_t tx0 = (bx & 0xffffu) / RT, tw = (bx >> 16) / RT - tx0 + 1u, ty0 = (by & 0xffffu) / RT;
-    uint32_t i = p - first;
-    uint32_t tile = (ty0 + i / tw) * tiles_x + tx0 + i % tw;
-    // neighbouring pairs often share a tile: one atomic for the lanes that do
-    const uint32_t lane = threadIdx.x & 31u, grp = __match_any_sync(__activemask(), tile), rank = __popc(grp & ((1u << lane) - 1u));
+    const uint32_t tile = listed ? (ty0 + i / tw) * tiles_x + tx0 + i % tw : 0xffffffffu;
+    // Pairs of neighbouring small triangles often share a tile: one atomic for the lanes that do.  A triangle's own tiles are
+    // distinct, so a warp of up to RS_SHARE triangles has little to share and skips the match, which takes a round for each
+    // distinct tile: with the match always, and from 4, 8 and 16 changes of triangle on, a room at 3840 x 2160 30, 16, 16, 16 us,
+    // 120k mixed triangles at 1920 x 1080 34, 24, 30, 32, 262k there 24, 25, 35, 65 (an atomic a pair: 16, 34, 66).
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, lo, 1);
+    const uint32_t changes = __popc(__ballot_sync(0xffffffffu, lane != 0u && prev != lo));
+    uint32_t grp = 1u << lane;
+    if (changes >= RS_SHARE) grp = __match_any_sync(0xffffffffu, tile);
+    const uint32_t rank = __popc(grp & ((1u << lane) - 1u));
     if (!FILL) {
-      if (rank == 0u) atomicAdd(&rd.tile_cnt[tile], (uint32_t)__popc(grp));
+      if (listed && rank == 0u) atomicAdd(&rd.tile_cnt[tile], (uint32_t)__popc(grp));
     } else {
       uint32_t slot = 0;
-      if (rank == 0u) slot = atomicAdd(&rd.tile_fill[tile], (uint32_t)__popc(grp));
-      slot = __shfl_sync(grp, slot, __ffs(grp) - 1) + rank;
-      rd.list[rd.tile_cnt[tile] + slot] = lo;
+      if (listed && rank == 0u) slot = atomicAdd(&rd.tile_fill[tile], (uint32_t)__popc(grp));
+      slot = __shfl_sync(0xffffffffu, slot, __ffs(grp) - 1) + rank;
+      if (listed) rd.list[rd.tile_cnt[tile] + slot] = lo;
     }
   }
 }

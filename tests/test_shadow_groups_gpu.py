@@ -1,6 +1,7 @@
 """The shadow raster's groups of chunks: a warp takes 1, 2, 4 or 8 consecutive 128-texel chunks by the number of chunks there
-are, crossing from triangle to triangle inside a group.  Scenes whose chunk totals lie on each side of the rule's lines (10, 1,484, 27,905, 47,442, 84,049 and
-241,963 chunks), of wide boxes, boxes of less than a chunk and triangles without any texel between them; every texel equals the oracle's map bit for bit."""
+are, crossing from triangle to triangle inside a group.  Scenes whose chunk totals lie on each side of the rule's lines (10,
+1,484, 27,905, 47,442, 84,049 and 241,963 chunks), of wide boxes, boxes of less than a chunk and triangles without any texel
+between them; every texel equals the oracle's map bit for bit."""
 import numpy as np
 import pytest
 
