@@ -290,17 +290,23 @@ __device__ __forceinline__ uint32_t block_min_256(uint32_t x, uint32_t *ws) {
 // (triangle, pixel) pairs go 256 at a time to the block's threads, the keys meeting in shared memory by atomic maxima (the
 // order of which does not matter).  With every triangle walked by all 256 threads a triangle of nine pixels cost as much as
 // one that fills the tile, and the whole chunk was sorted.  Bound by issue (81 % active, some 120 instructions a row of ray
-// tests): 262k triangles at 1920 x 1080 281 -> 203 us, at 1280 x 720 287 -> 135, 26k at 640 x 360 51 -> 27 (dealt over a warp
+// tests): 262k triangles at 1920 x 1080 282 -> 201 us, at 1280 x 720 274 -> 136, 26k at 640 x 360 51 -> 28 (dealt over a warp
 // instead of the block: 242, 143, 36).  Taking a long list or a chunk's small ones in bands of depth bound, nearest first,
 // pruned nothing (203 and 222 us).  Fragments of alpha-masked materials whose alpha falls below the cutoff are left out;
 // then the winner's depth, normal and style tag.
-constexpr uint32_t RS_SMALL = 96;   // 48: 211 us on the first of these, 144: 215
-__global__ void __launch_bounds__(256) k_rs_tiles(SceneDev s, const float *__restrict__ F, uint32_t W, uint32_t H,
+// RS_SMALL: boxes between a quarter and a third of a tile cost about the same either way where little hides them, but in a
+// scene many triangles deep the walk front to back leaves most of their pixels out.  With 64, 80 and 96: 262k triangles at
+// 1280 x 720 140, 136, 137 us, at 3840 x 2160 560, 576, 582; 300k mixed ones, deep, at 1920 x 1080 217, 229, 252 (209 with
+// every triangle walked); 25k at 640 x 360 30, 28, 27.  Five blocks an SM (the compiler alone takes 64 registers for four;
+// six spill): a room at 1920 x 1080 121 -> 114 us.
+constexpr uint32_t RS_SMALL = 80;
+__global__ void __launch_bounds__(256, 5) k_rs_tiles(SceneDev s, const float *__restrict__ F, uint32_t W, uint32_t H,
                                                   uint32_t tiles_x, RasterDev rd, float *depth, uint2 *normal,
                                                   uint8_t *tag) {
   grid_dep_wait();
   __shared__ float4 sa[256], se1[256], se2[256];
-  __shared__ uint32_t sval[256], s_large[256], s_order[256], s_first[256], s_geo[256];
+  __shared__ uint32_t sval[256], s_order[256], s_first[256], s_geo[256];
+  __shared__ __align__(16) uint32_t s_key[256];
   __shared__ float sdx[256], sdy[256], sdz[256];
   __shared__ unsigned long long s_best[256];
   __shared__ uint32_t ws[8], s_nlarge;
@@ -321,7 +327,8 @@ __global__ void __launch_bounds__(256) k_rs_tiles(SceneDev s, const float *__res
     for (uint32_t c0 = beg; c0 < end; c0 += 256u) {
       const uint32_t n = min(256u, end - c0);
       if (threadIdx.x == 0) s_nlarge = 0u;
-      uint32_t far = block_min_256(my_depth, ws);   // (also orders the line above and the last chunk's reads before what follows)
+      s_key[threadIdx.x] = 0u;
+      uint32_t far = block_min_256(my_depth, ws);   // (also orders the lines above and the last chunk's reads before what follows)
       // this thread's triangle: its record, its pixels in the tile
       uint32_t area = 0, wdt = 1, org0 = 0;
       if (threadIdx.x < n) {
@@ -338,19 +345,20 @@ __global__ void __launch_bounds__(256) k_rs_tiles(SceneDev s, const float *__res
           area = wdt * (ay1 - ay0 + 1u);
           org0 = (ay0 - Y0) * RT + (ax0 - X0);
         }
-        if (area > RS_SMALL) s_large[atomicAdd(&s_nlarge, 1u)] = threadIdx.x;
+        if (area > RS_SMALL) s_key[atomicAdd(&s_nlarge, 1u)] = (bound & ~255u) | threadIdx.x;
       }
       __syncthreads();
       const uint32_t nl = s_nlarge;
       if (nl != 0u) {
-        if (threadIdx.x < nl) {   // front to back: each finds its place among the others
-          const uint32_t me = s_large[threadIdx.x], kb = __float_as_uint(sa[me].w);
+        if (threadIdx.x < nl) {   // front to back, to 256 units in the last place of the bound: each finds its place among the others
+          const uint32_t mine = s_key[threadIdx.x];
           uint32_t rank = 0;
-          for (uint32_t j = 0; j < nl; j++) {
-            const uint32_t o = s_large[j], ko = __float_as_uint(sa[o].w);
-            rank += (ko > kb || (ko == kb && o < me)) ? 1u : 0u;
+#pragma unroll 1
+          for (uint32_t j = 0; j < nl; j += 4u) {
+            const uint4 k = *reinterpret_cast<const uint4 *>(s_key + j);
+            rank += (k.x > mine ? 1u : 0u) + (k.y > mine ? 1u : 0u) + (k.z > mine ? 1u : 0u) + (k.w > mine ? 1u : 0u);
           }
-          s_order[rank] = me;
+          s_order[rank] = mine & 255u;
         }
         __syncthreads();
         for (uint32_t j = 0; j < nl; j++) {
@@ -358,7 +366,7 @@ __global__ void __launch_bounds__(256) k_rs_tiles(SceneDev s, const float *__res
           const uint32_t i = s_order[j];
           const float4 a = sa[i];
           const uint32_t bd = __float_as_uint(a.w);
-          if (bd < far) break;                     // no pixel of the tile can take this or a later triangle
+          if ((bd | 255u) < far) break;            // no pixel of the tile can take this or a later triangle
           if (!inside || bd < my_depth) continue;  // this pixel cannot
           const float4 e1 = se1[i], e2 = se2[i];
           const uint32_t bx = __float_as_uint(e1.w), by = __float_as_uint(e2.w);
