@@ -209,10 +209,14 @@ struct TraceOut { f3 rad; float T; uint32_t lvl, ptr, bit, tin, steps; };
 //  * the whole warp calls it (lanes without a ray pass live = false), and its lanes meet again before the hits are shaded:
 //    left to themselves they shaded in 2.6 groups of 4.5 lanes a warp.
 // Bound by instruction issue at half-empty warps (12.6 steps a warp for 6 a ray; 131 M warp instructions against 147 M on
-// the colonnade, 69 % issue-active at 24 warps an SM).  Traces, before and after: colonnade 165 -> 163 us, its world probes
-// 94 -> 85, leak room 39 -> 32, textured room 43 -> 36, served 640 x 360 48 -> 40, bounce volumes 62 -> 53 and 88 -> 72.
-// Where the descriptors lie in global memory the walk gains nothing (batch of 8: 324 -> 340).  Nested loops for the two
-// kinds of step took 424 us on the colonnade, 64 registers by recomputing 172, dropping the meeting point 173.
+// the colonnade, 69 % issue-active at 24 warps an SM).  Traces, before and after: colonnade 165 -> 162 us, its world probes
+// 100 -> 90, leak room at 640 x 360 23 -> 20, textured room 43 -> 36, served 640 x 360 48 -> 40, bounce volumes 62 -> 53 and
+// 88 -> 72.  Where millions of short rays fill the chip it costs 2-7 %: a room at 1920 x 1080 with three cascades 55.5 -> 59.2,
+// a batch of 8 in f32 324 -> 339 (f16 and bf16 363 -> 338).  Neither registers nor the batch's descriptors are the cause: 64
+// registers (four blocks an SM) take 337 in the batch, 60.1 in the room and 175 on the colonnade, blocks of 128 threads, seven an
+// SM, 344, 58.2 and 165, descriptors staged in shared memory 345.  Nested loops for the two kinds of step took 424 us on the
+// colonnade, 64 registers by recomputing 172, dropping the meeting point 173; a return of warps without any ray to walk and the
+// entered cell without integer conversions 163.
 // inv_pre: the direction's 1 / d with tiny components clamped, tabulated with the directions (the same IEEE quotients), or
 // null to divide here.
 __device__ __forceinline__ bool brick_empty(uint32_t ptr) { return ptr >= GI_MARK && ptr != GI_DROP; }
@@ -605,9 +609,10 @@ __global__ void __launch_bounds__(256) k_rsort_scatter(RcDev r) {
 // walks are the longest; a queue that ended on them left SMs idle behind its last warps: 0.197 -> 0.170 ms on the
 // colonnade).  SORT: positions go through the walk-length order (rperm) and each ray's key is stored for the next
 // solve.  With the dynamic layer's read (chains of scattered reads) four blocks an SM, 64 registers, instead of the three that
-// the walk's registers alone give: 556 -> 521 us on the colonnade with 64 moving boxes, 247 -> 241 at 1280 x 720.
+// the walk's registers alone give: 556 -> 521 us on the colonnade with 64 moving boxes, 247 -> 241 at 1280 x 720; likewise in
+// the walk-length order, whose warps are full: 128 -> 124 on the colonnade.
 template <int A, bool DYN, bool SORT>
-__global__ void __launch_bounds__(256, DYN ? 4 : 0) k_trace(RcDev r, VoxDev v, uint32_t *ray_counter) {
+__global__ void __launch_bounds__(256, DYN || SORT ? 4 : 0) k_trace(RcDev r, VoxDev v, uint32_t *ray_counter) {
   grid_dep_wait();
   uint32_t lane = threadIdx.x & 31u;
   uint32_t steps_acc = 0, traces_acc = 0, cap_acc = 0;
