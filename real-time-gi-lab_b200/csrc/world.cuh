@@ -16,7 +16,7 @@
 //  * the trace is the persistent ray loop of the screen path over the rays of every cascade's live probes.
 
 constexpr uint32_t W_NONE = 0xffffffffu;
-constexpr uint32_t W_CELLS = 4;              // grid cells a gather warp stages at once
+constexpr uint32_t W_CELLS = 4;              // grid cells a gather warp stages
 constexpr uint32_t W_COMPACT_SLOTS = 2048;   // hash slots per compact block (8 a thread)
 
 // hash32 (rc.ts:248-250)
@@ -667,12 +667,25 @@ __global__ void __launch_bounds__(256) k_w_project_sh(RcDev r, WorldDev w) {
   }
 }
 
+// A c0 probe's SH as stored, and as k_w_gather_cells stages it: float4 0-6 (words 28-31 are 0)
 template <int A>
-__device__ __forceinline__ f3 w_eval_sh(const RcDev &r, uint32_t qi, const float y[9]) {
-  float v[32];
+struct ShStored {
+  const RcDev &r;
+  uint32_t qi;
+  __device__ __forceinline__ float4 operator[](int j) const { return sh_load<A>(r, (size_t)qi * 8u + j); }
+};
+struct ShStaged {
+  const float4 *sh;
+  __device__ __forceinline__ float4 operator[](int j) const { return sh[j]; }
+};
+
+// evalSH (rc.ts:819-829)
+template <class S>
+__device__ __forceinline__ f3 w_eval_sh(const S &sh, const float y[9]) {
+  float v[28];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const float4 sc = sh_load<A>(r, (size_t)qi * 8u + j);
+  for (int j = 0; j < 7; j++) {
+    const float4 sc = sh[j];
     v[4 * j] = sc.x; v[4 * j + 1] = sc.y; v[4 * j + 2] = sc.z; v[4 * j + 3] = sc.w;
   }
   f3 es = mk(0.0f, 0.0f, 0.0f);
@@ -681,12 +694,10 @@ __device__ __forceinline__ f3 w_eval_sh(const RcDev &r, uint32_t qi, const float
   return vmax(es, mk(0.0f, 0.0f, 0.0f));
 }
 
-// The L0 and L1 coefficients (basis order 0, y, z, x) of a probe's stored SH, added with weight wt (shL1 + shAdd,
-// rc.ts:831-840)
-template <int A>
-__device__ __forceinline__ void w_sh_l1_add(const RcDev &r, uint32_t qi, float wt, f3 &c0, f3 &cy, f3 &cz, f3 &cx) {
-  const float4 a = sh_load<A>(r, (size_t)qi * 8u), b = sh_load<A>(r, (size_t)qi * 8u + 1u),
-               c = sh_load<A>(r, (size_t)qi * 8u + 2u);
+// The L0 and L1 coefficients (basis order 0, y, z, x) of a probe's SH, added with weight wt (shL1 + shAdd, rc.ts:831-840)
+template <class S>
+__device__ __forceinline__ void w_sh_l1_add(const S &sh, float wt, f3 &c0, f3 &cy, f3 &cz, f3 &cx) {
+  const float4 a = sh[0], b = sh[1], c = sh[2];
   c0 = fma3(mk(a.x, a.y, a.z), wt, c0);
   cy = fma3(mk(a.w, b.x, b.y), wt, cy);
   cz = fma3(mk(b.z, b.w, c.x), wt, cz);
@@ -720,12 +731,92 @@ __device__ __forceinline__ ToonRecv toon_receive(f3 c0, f3 c1y, f3 c1z, f3 c1x, 
   return out;
 }
 
-// gatherWorld (rc.ts:880-927) with relocate 'voxel', one thread per pixel: the eight c0 probes of the pixel's grid cell, weighted
-// trilinearly and by the side of the surface they are on; the probes voxels hide are skipped
-// (retested from two voxels out when every probe is hidden).  Photoreal pixels left black count in words 72-79.
-// TAG (once the G-buffer carries style tags): toon pixels (tag > 0.75) also interpolate the L0/L1 coefficients and
+// gatherWorld (rc.ts:880-927): the eight c0 probes of the pixel's grid cell, weighted trilinearly and by the side of the surface
+// they are on.  TAG (once the G-buffer carries style tags): toon pixels (tag > 0.75) also interpolate the L0/L1 coefficients and
 // go through the receiving operator (the irradiance replaced when the frame's style.y > 0.5), alpha 2 + band + 2 when
 // the directional part is at least a tenth of the ambient; other tagged pixels (tag > 0.25) get alpha 2.
+struct WPixel {
+  f3 x, n, f;      // position, normal, place in the grid cell
+  i3 cell, org;
+  int lod;
+  float s0, tag;   // the grid's spacing; the style tag
+  bool toon;
+};
+template <bool TAG>
+__device__ __forceinline__ WPixel w_pixel(const RcDev &r, uint32_t px, uint32_t py, size_t q, float d) {
+  const float *F = r.frame;
+  WPixel p;
+  p.x = world_at(F, (int)px, (int)py, d);
+  const uint2 nn = r.normal[q];
+  p.n = mk(h2f(nn.x & 0xffffu), h2f(nn.x >> 16), h2f(nn.y & 0xffffu));
+  p.lod = w_lod_for(F, length3(p.x - mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2])));
+  p.s0 = w_spacing(F, p.lod, 0u);
+  const f3 gp = mk(p.x.x / p.s0, p.x.y / p.s0, p.x.z / p.s0);
+  p.cell = vfloori(gp);
+  p.org = w_origin(F, p.s0);
+  p.f = gp - vi2f(p.cell);
+  p.tag = TAG ? r.unorm8[r.tag[q]] : 0.0f;
+  p.toon = TAG && p.tag > 0.75f;
+  return p;
+}
+__device__ __forceinline__ float w_probe_weight(const WPixel &p, uint32_t k, f3 pp) {
+  const i3 o = w_corner(k);
+  const f3 tw = mk(o.x == 1 ? p.f.x : 1.0f - p.f.x, o.y == 1 ? p.f.y : 1.0f - p.f.y, o.z == 1 ? p.f.z : 1.0f - p.f.z);
+  const f3 dv = pp - p.x;
+  const float side = dot(p.n, dv) / mx(length3(dv), 1e-5f);
+  return (tw.x * tw.y * tw.z + 1e-4f) * ((side + 1.0f) * (side + 1.0f) * 0.25f + 0.02f);
+}
+// What a pixel's probes add up to: irradiance, weight, and on toon pixels the L0 / L1 coefficients
+struct WSum {
+  f3 e, l0, ly, lz, lx;
+  float ws;
+  __device__ __forceinline__ WSum() {
+    e = l0 = ly = lz = lx = mk(0.0f, 0.0f, 0.0f);
+    ws = 0.0f;
+  }
+  template <class S>
+  __device__ __forceinline__ void add(const S &sh, const float y[9], float wt, bool toon) {
+    e = fma3(w_eval_sh(sh, y), wt, e);
+    ws += wt;
+    if (toon) w_sh_l1_add(sh, wt, l0, ly, lz, lx);
+  }
+};
+// The pixel's probes looked up and read one by one, those that hide(k, probe, position, weight) left out
+template <int A, class H>
+__device__ __forceinline__ void w_add_probes(const RcDev &r, const WorldDev &w, const WPixel &p, const float y[9], WSum &s, H hide) {
+  for (uint32_t k = 0; k < 8u; k++) {
+    const i3 o = w_corner(k);
+    const uint32_t qi = w_lookup(w, 0u, w_key_at(mki(p.cell.x + o.x, p.cell.y + o.y, p.cell.z + o.z), p.org, p.lod));
+    if (qi == W_NONE) continue;
+    const f3 pp = ld3(r.probes[r.c[0].probe_off + qi].pos);
+    const float wt = w_probe_weight(p, k, pp);
+    if (hide(k, qi, pp, wt)) continue;
+    s.add(ShStored<A>{r, qi}, y, wt, p.toon);
+  }
+}
+template <bool TAG>
+__device__ __forceinline__ void w_receive(const float *__restrict__ F, const WPixel &p, const WSum &s, f3 &res, float &alpha) {
+  if (s.ws > 0.0f) res = s.e / s.ws;
+  if (TAG) {
+    if (p.toon && s.ws > 0.0f) {
+      const float iw = 1.0f / s.ws;
+      const ToonRecv tr = toon_receive(s.l0 * iw, s.ly * iw, s.lz * iw, s.lx * iw, p.n, F[F_STYLE + 2]);
+      if (F[F_STYLE + 1] > 0.5f) res = tr.e;
+      alpha = 2.0f + tr.band + (tr.contrast >= 0.1f ? 2.0f : 0.0f);
+    } else if (p.toon || p.tag > 0.25f) {
+      alpha = 2.0f;
+    }
+  }
+}
+template <int A>
+__device__ __forceinline__ void w_store(const RcDev &r, size_t q, f3 res, float alpha) {
+  if ((A == GI_ATLAS_F32 || r.f32_out) && !r.irr_f16) reinterpret_cast<float4 *>(r.irr)[q] = make_float4(res.x, res.y, res.z, alpha);
+  else reinterpret_cast<uint2 *>(r.irr)[q] = make_uint2((uint32_t)f2h(res.x) | ((uint32_t)f2h(res.y) << 16),
+                                                       (uint32_t)f2h(res.z) | ((uint32_t)f2h(alpha) << 16));
+}
+
+// With relocate 'voxel', one thread per pixel: the probes voxels hide are skipped (retested from two voxels out when every probe
+// is hidden).  Photoreal pixels left black count in words 72-79.
 template <int A, bool TAG>
 __global__ void __launch_bounds__(256) k_w_gather(RcDev r, VoxDev v, WorldDev w) {
   grid_dep_wait();
@@ -735,210 +826,116 @@ __global__ void __launch_bounds__(256) k_w_gather(RcDev r, VoxDev v, WorldDev w)
   const uint32_t px = blockIdx.x * 16u + (wp & 3u) * 4u + (lane & 3u), py = blockIdx.y * 16u + (wp >> 2) * 8u + (lane >> 2);
   if (px >= r.width || py >= r.height) return;
   const size_t q = (size_t)py * r.width + px;
-  const float *F = r.frame;
   const float d = r.depth[q];
   f3 res = mk(0.0f, 0.0f, 0.0f);
   float alpha = 0.0f;
   bool black = false;
   if (d > 0.0f) {
     alpha = 1.0f;
-    const f3 x = world_at(F, (int)px, (int)py, d);
-    const uint2 nn = r.normal[q];
-    const f3 n = mk(h2f(nn.x & 0xffffu), h2f(nn.x >> 16), h2f(nn.y & 0xffffu));
-    const int lod = w_lod_for(F, length3(x - mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2])));
-    const float s0 = w_spacing(F, lod, 0u);
-    const f3 gp = mk(x.x / s0, x.y / s0, x.z / s0);
-    const i3 bb = vfloori(gp), org0 = w_origin(F, s0);
-    const f3 f = gp - vi2f(bb);
-    const uint32_t Lo = vox_level_for(v, vox_level(v, r, s0, 0u), x);
-    const f3 xo1 = x + n * (1.0f * vox_size(v, Lo));
+    const WPixel p = w_pixel<TAG>(r, px, py, q, d);
+    const uint32_t Lo = vox_level_for(v, vox_level(v, r, p.s0, 0u), p.x);
+    const f3 xo1 = p.x + p.n * (1.0f * vox_size(v, Lo));
     float y[9];
-    sh_basis(n, y);
-    f3 e = mk(0.0f, 0.0f, 0.0f);
-    float ws = 0.0f, ww[8];
+    sh_basis(p.n, y);
+    WSum s;
+    float ww[8];
     uint32_t hidden = 0, qq[8];
-    const float tagA = TAG ? r.unorm8[r.tag[q]] : 0.0f;
-    const bool toon = TAG && tagA > 0.75f;
-    f3 l0 = mk(0.0f, 0.0f, 0.0f), ly = l0, lz = l0, lx = l0;   // toon pixels: the L0 / L1 sums
-    for (uint32_t k = 0; k < 8u; k++) {
-      const i3 o = w_corner(k);
-      const uint32_t qi = w_lookup(w, 0u, w_key_at(mki(bb.x + o.x, bb.y + o.y, bb.z + o.z), org0, lod));
-      if (qi == W_NONE) continue;
-      const f3 tw = mk(o.x == 1 ? f.x : 1.0f - f.x, o.y == 1 ? f.y : 1.0f - f.y, o.z == 1 ? f.z : 1.0f - f.z);
-      const f3 pp = ld3(r.probes[r.c[0].probe_off + qi].pos);
-      const f3 dv = pp - x;
-      const float side = dot(n, dv) / mx(length3(dv), 1e-5f);
-      const float wt = (tw.x * tw.y * tw.z + 1e-4f) * ((side + 1.0f) * (side + 1.0f) * 0.25f + 0.02f);
-      if (w_seg_occluded(v, xo1, pp, Lo)) { hidden |= 1u << k; ww[k] = wt; qq[k] = qi; continue; }
-      e = fma3(w_eval_sh<A>(r, qi, y), wt, e);
-      ws += wt;
-      if (toon) w_sh_l1_add<A>(r, qi, wt, l0, ly, lz, lx);
-    }
-    if (ws <= 0.0f && hidden != 0u) {
-      const f3 xo2 = x + n * (2.0f * vox_size(v, Lo));
+    w_add_probes<A>(r, w, p, y, s, [&](uint32_t k, uint32_t qi, f3 pp, float wt) {
+      if (!w_seg_occluded(v, xo1, pp, Lo)) return false;
+      hidden |= 1u << k; ww[k] = wt; qq[k] = qi;
+      return true;
+    });
+    if (s.ws <= 0.0f && hidden != 0u) {
+      const f3 xo2 = p.x + p.n * (2.0f * vox_size(v, Lo));
       for (uint32_t k = 0; k < 8u; k++) {
         if ((hidden & (1u << k)) == 0u) continue;
         if (w_seg_occluded(v, xo2, ld3(r.probes[r.c[0].probe_off + qq[k]].pos), Lo)) continue;
-        e = fma3(w_eval_sh<A>(r, qq[k], y), ww[k], e);
-        ws += ww[k];
-        if (toon) w_sh_l1_add<A>(r, qq[k], ww[k], l0, ly, lz, lx);
+        s.add(ShStored<A>{r, qq[k]}, y, ww[k], p.toon);
       }
     }
-    black = ws <= 0.0f && hidden != 0u && tagA <= 0.25f;
-    if (ws > 0.0f) res = e / ws;
-    if (TAG) {
-      if (toon && ws > 0.0f) {
-        const float iw = 1.0f / ws;
-        const ToonRecv tr = toon_receive(l0 * iw, ly * iw, lz * iw, lx * iw, n, F[F_STYLE + 2]);
-        if (F[F_STYLE + 1] > 0.5f) res = tr.e;
-        alpha = 2.0f + tr.band + (tr.contrast >= 0.1f ? 2.0f : 0.0f);
-      } else if (toon || tagA > 0.25f) {
-        alpha = 2.0f;
-      }
-    }
+    black = s.ws <= 0.0f && hidden != 0u && p.tag <= 0.25f;
+    w_receive<TAG>(r.frame, p, s, res, alpha);
   }
   // black pixels: one atomic per counter word among the warp's lanes
   const unsigned act = __activemask();
   const unsigned grp = __match_any_sync(act, black ? (px & 7u) : 8u);
   if (black && (uint32_t)(__ffs(grp) - 1) == (threadIdx.x & 31u)) atomicAdd(&r.counts[72 + (px & 7u)], (uint32_t)__popc(grp));
-  if ((A == GI_ATLAS_F32 || r.f32_out) && !r.irr_f16) reinterpret_cast<float4 *>(r.irr)[q] = make_float4(res.x, res.y, res.z, alpha);
-  else reinterpret_cast<uint2 *>(r.irr)[q] = make_uint2((uint32_t)f2h(res.x) | ((uint32_t)f2h(res.y) << 16),
-                                                       (uint32_t)f2h(res.z) | ((uint32_t)f2h(alpha) << 16));
+  w_store<A>(r, q, res, alpha);
 }
 
-// evalSH (rc.ts:819-829) of a probe's SH as staged (float4 0-6)
-__device__ __forceinline__ f3 w_eval_sh_at(const float4 *__restrict__ sh, const float y[9]) {
-  float v[28];
-#pragma unroll
-  for (int j = 0; j < 7; j++) {
-    const float4 sc = sh[j];
-    v[4 * j] = sc.x; v[4 * j + 1] = sc.y; v[4 * j + 2] = sc.z; v[4 * j + 3] = sc.w;
-  }
-  f3 es = mk(0.0f, 0.0f, 0.0f);
-#pragma unroll
-  for (int k = 0; k < 9; k++) es = fma3(mk(v[3 * k], v[3 * k + 1], v[3 * k + 2]), y[k], es);
-  return vmax(es, mk(0.0f, 0.0f, 0.0f));
-}
-
-// The L0 and L1 coefficients (basis order 0, y, z, x) of a probe's staged SH, added with weight wt (shL1 + shAdd,
-// rc.ts:831-840)
-__device__ __forceinline__ void w_sh_l1_add_at(const float4 *__restrict__ sh, float wt, f3 &c0, f3 &cy, f3 &cz, f3 &cx) {
-  const float4 a = sh[0], b = sh[1], c = sh[2];
-  c0 = fma3(mk(a.x, a.y, a.z), wt, c0);
-  cy = fma3(mk(a.w, b.x, b.y), wt, cy);
-  cz = fma3(mk(b.z, b.w, c.x), wt, cz);
-  cx = fma3(mk(c.y, c.z, c.w), wt, cx);
-}
-
-// gatherWorld where no probe can be hidden (relocate 'gbuffer' or 'none'): the warp's distinct grid cells are looked up and
-// their probes' positions and SH staged in shared memory once, four cells a round.  The lanes of a warp share a few cells, and
-// each looking up and loading its own eight probes (72 dependent 128-bit loads a pixel) waited on them: 97 -> 74 us for a
-// room at 1280 x 720 in f16.  With voxel relocation the segment tests are most of the work and a warp with more than four
-// cells would run them once a round: staged 375 us against 366 on the colonnade at 1920 x 1080, so that keeps k_w_gather.
+// Where no probe can be hidden (relocate 'gbuffer' or 'none'): the warp's distinct grid cells are looked up and their probes'
+// positions and SH staged in shared memory once.  The lanes of a warp share a few cells, and each looking up and loading its own
+// eight probes (72 dependent 128-bit loads a pixel) waited on them: 95 -> 63 us for a room at 1280 x 720 in f16, 216 -> 130 for
+// the colonnade at 1920 x 1080.  A warp of more than four cells has little to share and reads its probes one by one: taking its
+// cells four a round ran the weights once a round with a few lanes each, 26 us for 17 with cells of 8 pixels at 256 x 144
+// (16.99 now).  With voxel relocation the segment tests are most of the work and k_w_gather reads its probes one by one: staged
+// 375 us against 366 on the colonnade at 1920 x 1080.
 template <int A, bool TAG>
 __global__ void __launch_bounds__(256, 4) k_w_gather_cells(RcDev r, WorldDev w) {
   grid_dep_wait();
-  // per warp up to four grid cells' eight probes: the stored SH in float4 0-6, the position in 7 (SH words 28-31 are 0)
+  // per warp up to four grid cells' eight probes: the stored SH in float4 0-6, the position in 7
   __shared__ float4 s_cell[8][W_CELLS][8][8];
   __shared__ uint32_t s_probe[8][W_CELLS][8];
-  // a warp takes a 4 x 8 tile of the block's 16 x 16 pixels (neighbouring pixels share probes and segment lengths;
-  // 0.378 ms on the colonnade with 16 x 2 rows, 0.360 with 8 x 4 tiles, 0.354 with 4 x 8, 0.360 with 2 x 16)
+  // a warp takes a 4 x 8 tile of the block's 16 x 16 pixels, as in k_w_gather
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const uint32_t px = blockIdx.x * 16u + (wp & 3u) * 4u + (lane & 3u), py = blockIdx.y * 16u + (wp >> 2) * 8u + (lane >> 2);
   const bool on = px < r.width && py < r.height;
   const size_t q = on ? (size_t)py * r.width + px : 0u;
-  const float *F = r.frame;
   const float d = on ? r.depth[q] : 0.0f;
   const bool live = d > 0.0f;
   f3 res = mk(0.0f, 0.0f, 0.0f);
   float alpha = live ? 1.0f : 0.0f;
-  f3 x = mk(0.0f, 0.0f, 0.0f), n = x, f = x;
-  i3 bb = mki(0, 0, 0), org0 = bb;
-  int lod = 0;
-  float s0 = 1.0f;
-  if (live) {
-    x = world_at(F, (int)px, (int)py, d);
-    const uint2 nn = r.normal[q];
-    n = mk(h2f(nn.x & 0xffffu), h2f(nn.x >> 16), h2f(nn.y & 0xffffu));
-    lod = w_lod_for(F, length3(x - mk(F[F_EYE], F[F_EYE + 1], F[F_EYE + 2])));
-    s0 = w_spacing(F, lod, 0u);
-    const f3 gp = mk(x.x / s0, x.y / s0, x.z / s0);
-    bb = vfloori(gp);
-    org0 = w_origin(F, s0);
-    f = gp - vi2f(bb);
-  }
-  // The warp's distinct cells, up to four a round (nearly always all of them): lane 8 g + k looks corner k of cell g up, the
-  // lanes load the cells' probes into shared memory together, and each pixel reads its own cell's there.
-  for (unsigned rem = __ballot_sync(0xffffffffu, live); rem != 0u;) {
-    int mine = -1, lead = (int)lane;
-    uint32_t cells = 0;
+  WPixel p;
+  p.cell = p.org = mki(0, 0, 0);
+  p.lod = 0;
+  if (live) p = w_pixel<TAG>(r, px, py, q, d);
+  // the warp's distinct cells, up to four
+  unsigned rem = __ballot_sync(0xffffffffu, live);
+  int mine = 0, lead = (int)lane;
+  uint32_t cells = 0;
 #pragma unroll
-    for (uint32_t g = 0; g < W_CELLS; g++) {
-      if (rem == 0u) break;
-      const int src = __ffs(rem) - 1;
-      const int sx = __shfl_sync(0xffffffffu, bb.x, src), sy = __shfl_sync(0xffffffffu, bb.y, src),
-                sz = __shfl_sync(0xffffffffu, bb.z, src), sl = __shfl_sync(0xffffffffu, lod, src);   // by every lane
-      const bool same = sx == bb.x && sy == bb.y && sz == bb.z && sl == lod;
-      const unsigned grp = __ballot_sync(0xffffffffu, same) & rem;
-      if ((grp >> lane) & 1u) mine = (int)g;
-      if ((lane >> 3) == g) lead = src;
-      rem &= ~grp;
-      cells = g + 1u;
-    }
-    {
-      const i3 cb = mki(__shfl_sync(0xffffffffu, bb.x, lead), __shfl_sync(0xffffffffu, bb.y, lead), __shfl_sync(0xffffffffu, bb.z, lead));
-      const i3 co = mki(__shfl_sync(0xffffffffu, org0.x, lead), __shfl_sync(0xffffffffu, org0.y, lead), __shfl_sync(0xffffffffu, org0.z, lead));
-      const int cl = __shfl_sync(0xffffffffu, lod, lead);
-      const i3 o = w_corner(lane & 7u);
-      if ((lane >> 3) < cells)
-        s_probe[wp][lane >> 3][lane & 7u] = w_lookup(w, 0u, w_key_at(mki(cb.x + o.x, cb.y + o.y, cb.z + o.z), co, cl));
-    }
+  for (uint32_t g = 0; g < W_CELLS; g++) {
+    if (rem == 0u) break;
+    const int src = __ffs(rem) - 1;
+    const int sx = __shfl_sync(0xffffffffu, p.cell.x, src), sy = __shfl_sync(0xffffffffu, p.cell.y, src),
+              sz = __shfl_sync(0xffffffffu, p.cell.z, src), sl = __shfl_sync(0xffffffffu, p.lod, src);   // by every lane
+    const bool same = sx == p.cell.x && sy == p.cell.y && sz == p.cell.z && sl == p.lod;
+    const unsigned grp = __ballot_sync(0xffffffffu, same) & rem;
+    if ((grp >> lane) & 1u) mine = (int)g;
+    if ((lane >> 3) == g) lead = src;
+    rem &= ~grp;
+    cells = g + 1u;
+  }
+  float y[9];
+  if (live) sh_basis(p.n, y);
+  WSum s;
+  if (rem == 0u) {
+    // lane 8 g + k looks corner k of cell g up, the lanes load the cells' probes into shared memory together, and each pixel
+    // reads its own cell's there
+    const i3 cb = mki(__shfl_sync(0xffffffffu, p.cell.x, lead), __shfl_sync(0xffffffffu, p.cell.y, lead), __shfl_sync(0xffffffffu, p.cell.z, lead));
+    const i3 co = mki(__shfl_sync(0xffffffffu, p.org.x, lead), __shfl_sync(0xffffffffu, p.org.y, lead), __shfl_sync(0xffffffffu, p.org.z, lead));
+    const int cl = __shfl_sync(0xffffffffu, p.lod, lead);
+    const i3 o = w_corner(lane & 7u);
+    if ((lane >> 3) < cells)
+      s_probe[wp][lane >> 3][lane & 7u] = w_lookup(w, 0u, w_key_at(mki(cb.x + o.x, cb.y + o.y, cb.z + o.z), co, cl));
     __syncwarp();
     for (uint32_t i = lane; i < cells * 64u; i += 32u) {
       const uint32_t g = i >> 6, k = (i >> 3) & 7u, j = i & 7u, qi = s_probe[wp][g][k];
       if (qi != W_NONE) s_cell[wp][g][k][j] = j < 7u ? sh_load<A>(r, (size_t)qi * 8u + j) : r.probes[r.c[0].probe_off + qi].pos;
     }
     __syncwarp();
-    if (mine >= 0) {
+    if (live) {
       const float4 (*cell)[8] = s_cell[wp][mine];
-      const uint32_t *probe = s_probe[wp][mine];
-      float y[9];
-      sh_basis(n, y);
-      f3 e = mk(0.0f, 0.0f, 0.0f);
-      float ws = 0.0f;
-      const float tagA = TAG ? r.unorm8[r.tag[q]] : 0.0f;
-      const bool toon = TAG && tagA > 0.75f;
-      f3 l0 = mk(0.0f, 0.0f, 0.0f), ly = l0, lz = l0, lx = l0;   // toon pixels: the L0 / L1 sums
       for (uint32_t k = 0; k < 8u; k++) {
-        const i3 o = w_corner(k);
-        if (probe[k] == W_NONE) continue;
-        const f3 tw = mk(o.x == 1 ? f.x : 1.0f - f.x, o.y == 1 ? f.y : 1.0f - f.y, o.z == 1 ? f.z : 1.0f - f.z);
-        const f3 pp = ld3(cell[k][7]);
-        const f3 dv = pp - x;
-        const float side = dot(n, dv) / mx(length3(dv), 1e-5f);
-        const float wt = (tw.x * tw.y * tw.z + 1e-4f) * ((side + 1.0f) * (side + 1.0f) * 0.25f + 0.02f);
-        e = fma3(w_eval_sh_at(cell[k], y), wt, e);
-        ws += wt;
-        if (toon) w_sh_l1_add_at(cell[k], wt, l0, ly, lz, lx);
-      }
-      if (ws > 0.0f) res = e / ws;
-      if (TAG) {
-        if (toon && ws > 0.0f) {
-          const float iw = 1.0f / ws;
-          const ToonRecv tr = toon_receive(l0 * iw, ly * iw, lz * iw, lx * iw, n, F[F_STYLE + 2]);
-          if (F[F_STYLE + 1] > 0.5f) res = tr.e;
-          alpha = 2.0f + tr.band + (tr.contrast >= 0.1f ? 2.0f : 0.0f);
-        } else if (toon || tagA > 0.25f) {
-          alpha = 2.0f;
-        }
+        if (s_probe[wp][mine][k] == W_NONE) continue;
+        s.add(ShStaged{cell[k]}, y, w_probe_weight(p, k, ld3(cell[k][7])), p.toon);
       }
     }
-    if (rem != 0u) __syncwarp();   // the next round's cells overwrite these
+  } else if (live) {   // more than four cells: little is shared
+    w_add_probes<A>(r, w, p, y, s, [](uint32_t, uint32_t, f3, float) { return false; });
   }
-  if (!on) return;
-  if ((A == GI_ATLAS_F32 || r.f32_out) && !r.irr_f16) reinterpret_cast<float4 *>(r.irr)[q] = make_float4(res.x, res.y, res.z, alpha);
-  else reinterpret_cast<uint2 *>(r.irr)[q] = make_uint2((uint32_t)f2h(res.x) | ((uint32_t)f2h(res.y) << 16),
-                                                       (uint32_t)f2h(res.z) | ((uint32_t)f2h(alpha) << 16));
+  if (live) w_receive<TAG>(r.frame, p, s, res, alpha);
+  if (on) w_store<A>(r, q, res, alpha);
 }
 
 // One world-probe solve (Rc.encode, rc.ts:1180-1221): giBuild (clear .. linkParents), giTrace (the bounce volume, the
