@@ -286,7 +286,7 @@ struct VoxDev {
   float v0;
   uint32_t levels, G, max_bricks, max_voxels, big_cap;
   uint32_t chunk_log2, blocks;   // tuning: cells per big-triangle work item (log2), resident blocks per SM
-  uint32_t citem_cap, scan_cap;  // entries of citem (0: no table); blocks the chained scans may take
+  uint32_t citem_cap, scan_cap;  // entries of citem (0: no table); parts the chained scans may have (gi_launch_vox_build refuses more)
   float vs[8];         // voxel size per level, ldexpf(v0, L) (vox_derived)
   int32_t lim_vox[8], lim_brick[8];   // voxRange's limit f2i(G * size * 8 / cell), voxel and brick cells (vox_derived)
   int32_t origin[8][4];

@@ -29,7 +29,11 @@ namespace {
 
 constexpr uint32_t NOALLOC_MAX_BRICKS = 4096;          // representative table: 4096 x 512 words = 8 MiB
 constexpr uint32_t NOALLOC_BIG_CAP = 1u << 16;         // per big-triangle list: 16 x 65536 words = 4 MiB
-constexpr uint32_t NOALLOC_SCAN_WORDS = 1u << 14;      // chained-scan blocks: levels * G^3 <= 2^25 pointers
+constexpr uint32_t NOALLOC_MAX_POINTERS = 1u << 25;    // levels * G^3: two levels of the largest clipmap
+// the chained scans' parts: the brick allocation takes 256 pointers a part up to 8,192 pointers, 1,024 up to 524,288 and 4,096
+// above (at most 8,192 parts), the voxel allocation 256 bricks a part
+constexpr uint32_t NOALLOC_SCAN_WORDS = 1u << 14;
+static_assert(NOALLOC_MAX_POINTERS / 4096u <= NOALLOC_SCAN_WORDS && NOALLOC_MAX_BRICKS / 256u <= NOALLOC_SCAN_WORDS, "scan parts");
 // the chained scans' states (64-bit words) start on an even word
 constexpr uint32_t NOALLOC_LOOK_AT = (NOALLOC_MAX_BRICKS * 512u + 16u * NOALLOC_BIG_CAP + NOALLOC_MAX_BRICKS + 1u + 4u +
                                       8u * NOALLOC_BIG_CAP + 1u) & ~1u;
@@ -96,9 +100,9 @@ extern "C" int gi_vox_build_noalloc(const gi_vox_params *p, const double eye[3],
     return fail(GI_ERR_INVALID, "gi_vox_build_noalloc: max_bricks %u exceeds the static scratch (at most %u bricks)",
                 p->max_bricks, NOALLOC_MAX_BRICKS);
   uint64_t nptr = (uint64_t)p->levels * p->G * p->G * p->G;
-  if ((nptr + 2047u) / 2048u > NOALLOC_SCAN_WORDS)
+  if (nptr > NOALLOC_MAX_POINTERS)
     return fail(GI_ERR_INVALID, "gi_vox_build_noalloc: levels * G^3 = %llu pointers exceeds the static scratch (at most %u)",
-                (unsigned long long)nptr, NOALLOC_SCAN_WORDS * 2048u);
+                (unsigned long long)nptr, NOALLOC_MAX_POINTERS);
   if (p->max_voxels < 1 || p->max_voxels >= (1u << 31)) return fail(GI_ERR_INVALID, "gi_vox_build_noalloc: max_voxels %u", p->max_voxels);
   for (int a = 0; a < 3; a++)
     if (!isfinite(eye[a])) return fail(GI_ERR_INVALID, "gi_vox_build_noalloc: eye is not finite");

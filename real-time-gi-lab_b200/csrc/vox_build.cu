@@ -870,9 +870,10 @@ cudaError_t gi_launch_vox_build(const VoxDev &v, const SceneDev &s, uint32_t sm_
   uint32_t persist = sm_count * v.blocks;   // blocks of 256 threads per SM for the grid-stride passes (default 8)
   // Pointers per thread of the brick allocation: 1 while the parts are at most one look-back step (32 parts), 4 to some 500
   // parts, 16 above (measured: 512 pointers 4.2 us with 1, 8.5 with 16; 16,384: 6.0 with 1, 5.6 with 4, 9.2 with 16; 163,840:
-  // 10.6 with 1, 8.0 with 4; 1.3 M: 11.4 with 16).  The parts of both chained scans fit the scan words, allotted for 256 a part.
+  // 10.6 with 1, 8.0 with 4; 1.3 M: 14.1 with 4, 12.2 with 16; 2.1 M: 19 to 22, 13 to 15; 16.8 M: 125, 46).
   const uint32_t E = nptr <= 8192u ? 1u : (nptr <= 524288u ? 4u : 16u);
   const uint32_t ab = (nptr + 256u * E - 1u) / (256u * E), vb = (v.max_bricks + VOX_CHUNK - 1u) / VOX_CHUNK;
+  if (max(ab, vb) > v.scan_cap) return cudaErrorInvalidValue;   // the scans' states would run past v.look
   GI_TRY(gi_launch(k_clear, min((nptr + 255u) / 256u + 1u, persist), 256, st, v, ab));
   uint32_t tb = (s.threads + 255u) / 256u;   // threads of the triangle passes (the work items' triangles)
   if (tb) GI_TRY(gi_launch(k_mark_bricks, tb, 256, st, v, s));
