@@ -102,3 +102,12 @@ def test_ranges(rule, lo, hi):
     bad, through = rule(x.view(np.float32), _divisors(rng, 25))
     assert bad == 0
     assert through > 0
+
+
+@pytest.mark.parametrize("m", [0x000000, 0x000001, 0x7fffff, 0x7ffffe, 0x555555, 0x4ccccd, 0x6dbb5a])
+def test_binade(rule, m):
+    """A whole binade of numerators (three in a vector) for one divisor: the hard cases of the last rounding are among them."""
+    x = np.arange(0x3f800000, 0x40000000, dtype=np.uint32)[:(1 << 23) // 3 * 3]
+    bad, through = rule(x.view(np.float32), np.array([(127 << 23) | m], np.uint32).view(np.float32))
+    assert bad == 0
+    assert through == x.size // 3
