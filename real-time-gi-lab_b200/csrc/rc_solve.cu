@@ -97,7 +97,8 @@ __device__ __forceinline__ float smoothstep_(float e0, float e1, float x) {
 // around q that are active, on that side and whose reach along their axes covers q.  The four texels
 // that the tests read are in flight together, the three that are summed only behind them: with each read behind the test
 // before it, the waits were most of bn_rays (1600x900 73 -> 67 us, 1280x720 52 -> 50 us) and of a small bnInject (24.5 ->
-// 20.5 us); with all seven ahead, bnInject at 1600x900, where instructions bind, took 77 us for 70.
+// 20.5 us); over 25 scenes and clipmaps bnInject takes 8 % less, and where the voxels of 300k triangles fill its pool, and
+// instructions bind, 4 to 7 % more (105 -> 112 us).  With all seven ahead it took 77 us for 70 at 1600x900.
 __device__ f3 bn_read(const BounceDev &b, const uint2 *vol, f3 q, f3 p, f3 n) {
   const i3 org = bn_origin(b, vol);
   const f3 g = mk(q.x / b.cell, q.y / b.cell, q.z / b.cell) - vi2f(org);

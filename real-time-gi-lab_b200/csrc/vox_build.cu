@@ -431,8 +431,10 @@ __device__ __forceinline__ void voxelize_one(const VoxDev &v, const SceneDev &s,
   atomicMax(&v.rep[ri], t + 1u);
 }
 
-// Big items of at most this many cells go to k_vox_bits_big in groups (vox_medium), larger ones in chunks
-// (a cylinder facet of 44 cells, the colonnade's usual one, does better as a chunk of its own: 29 us against 37 with 64 here)
+// Big items of at most this many cells go to k_vox_bits_big in groups (vox_medium), larger ones in chunks.  Both passes of
+// voxBits over six scenes and twelve clipmaps: with 16 4 % longer (up to 37 %: a colonnade in one level of 1024^3); with 64 1 %
+// shorter, but a colonnade's facets of 44 cells do better as chunks of their own (72 us against 78 at 4 x 128^3, 104 against 114
+// at 5 x 256^3).
 constexpr uint32_t VOX_MEDIUM = 32, MEDIUM_GROUP = 8;
 
 // The large items' work for k_vox_bits_big: every (triangle, level) of voxBits with more cells is cut into chunks of
