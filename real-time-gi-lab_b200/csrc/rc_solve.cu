@@ -213,9 +213,10 @@ struct TraceOut { f3 rad; float T; uint32_t lvl, ptr, bit, tin, steps; };
 // the colonnade, 69 % issue-active at 24 warps an SM).  Traces, before and after: colonnade 165 -> 162 us, its world probes
 // 100 -> 90, leak room at 640 x 360 23 -> 20, textured room 43 -> 36, served 640 x 360 48 -> 40, bounce volumes 62 -> 53 and
 // 88 -> 72.  Where millions of short rays fill the chip it costs 2-7 %: a room at 1920 x 1080 with three cascades 55.5 -> 59.2,
-// a batch of 8 in f32 324 -> 339 (f16 and bf16 363 -> 338).  Neither registers nor the batch's descriptors are the cause: 64
+// a batch of 8 in f32 324 -> 339 (f16 and bf16 363 -> 338): in that room 43.6 M warp instructions against 42.3 M, a longer set-up
+// that a walk of one or two steps does not win back, at 36 % of warps active against 48 %.  More warps alone do not help: 64
 // registers (four blocks an SM) take 337 in the batch, 60.1 in the room and 175 on the colonnade, blocks of 128 threads, seven an
-// SM, 344, 58.2 and 165, descriptors staged in shared memory 345.  Nested loops for the two kinds of step took 424 us on the
+// SM, 344, 58.2 and 165; nor do the batch's descriptors staged in shared memory, 345.  Nested loops for the two kinds of step took 424 us on the
 // colonnade, 64 registers by recomputing 172, dropping the meeting point 173; a return of warps without any ray to walk and the
 // entered cell without integer conversions 163.
 // inv_pre: the direction's 1 / d with tiny components clamped, tabulated with the directions (the same IEEE quotients), or
